@@ -28,7 +28,7 @@ size_t engine_smem_bytes();
 cudaError_t launch_mother(float fb, int N, float norm, float* out, cudaStream_t st);
 cudaError_t launch_twiddle(int log2N, float2* tw, cudaStream_t st);
 cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log2N, const float2* tw,
-                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels);
+                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R);
 cudaError_t launch_forward_batched(const FwdJob* jobs, int njobs, int log2N, const float2* tw, cudaStream_t st,
                                    int* n_kernels, bool real);
 cudaError_t launch_inverse_batched(const FwdJob* jobs, int njobs, int log2N, const float2* tw, cudaStream_t st,
@@ -49,8 +49,11 @@ cudaError_t launch_engine(const EngineParams& p, const CUtensorMap& omap, int gr
 cudaError_t tc_configure();
 cudaError_t launch_tc_weights(const SigDesc* sigs, const RowDesc* rows, const int* row_list, int n_list,
                               const float* pool, float* wts, cudaStream_t st);
-cudaError_t launch_tc(const TcParams& p, const CUtensorMap& omap, int out_type, int grid, cudaStream_t st);
-cudaError_t launch_shift_spectrum(const float2* X, int log2N, float2* J, cudaStream_t st);
+size_t tc_table_bytes();
+int tc_table_blocks(int log2M);
+cudaError_t launch_tc_tables(int log2M, int KC, int log2R, unsigned char* out, cudaStream_t st);
+cudaError_t launch_tc(const TcParams& p, int log2R, int out_type, int grid, cudaStream_t st);
+cudaError_t launch_shift_spectrum(const float2* X, int log2N, float2* J, float2* Jp, int log2R, cudaStream_t st);
 cudaError_t launch_align_spill(const SigDesc* sigs, const RowDesc* rows, const int* list, int nlist,
                                const float* pool, float2* out, int n, float extra, cudaStream_t st);
 cudaError_t launch_doublesided_combine(float2* out, const float2* V, long long rows, int n, int dec, int log2N,
@@ -247,6 +250,8 @@ struct PlanSignal {
     int row0 = 0;        // global index of its first produced row
     int table = 0;       // index into fcwt_plan::tables
     DevBuf X;            // forward spectrum, N complex
+    int log2R = 0;       // tensor-core rows: P2 = 16 << log2R (0: the signal has none)
+    DevBuf Xp;           // tensor-core rows: bins < N/2 in perm_bin order
 };
 
 // Tables shared by all signals of one padded length.
@@ -261,11 +266,10 @@ struct fcwt_plan {
     bool is_complex = false;
     std::vector<PlanSignal> sig;
     std::vector<PlanTables> tables;
-    DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, tc_wts;
+    DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, tc_wts, tc_tabs;
     DevBuf tc_units;  // work list of the tensor-core engine (rows, the last ones possibly split)
-    int n_units = 0;
-    // Per-execution uploads of batched plans (forward jobs, per-output tensor
-    // maps) go through a ring of pinned host slots; a slot is rewritten only
+    int n_units[2] = {0, 0};  // units of R = 16 and, after them, of R = 8
+    // Per-execution uploads of batched plans (forward jobs) go through a ring of pinned host slots; a slot is rewritten only
     // after the copy that read it has run (its event), so back-to-back
     // executions with different buffers never see each other's data.
     struct UploadSlot {
@@ -276,8 +280,6 @@ struct fcwt_plan {
     };
     std::array<UploadSlot, 4> uploads;
     int upload_next = 0;
-    DevBuf tmaps, graph_tmaps;               // per-output tensor maps (batched plans), device copies
-    std::array<unsigned long long, fcwt::kMaxOuts / 64> graph_tmap_mask{};
     int n_items = 0;
     int n_rows = 0;
     int n_tc = 0;  // rows run by the tensor-core engine
@@ -287,7 +289,7 @@ struct fcwt_plan {
     bool compat_align = false; // reference's odd-n row shift (FCWT_COMPAT_ALIGN)
     DevBuf shifted;            // compat_align: the rows written one sample to the right
     int n_shifted = 0;
-    DevBuf Xs, sigs2, ds_tmp;  // doublesided: shifted spectrum, its signal descriptor, second-pass rows
+    DevBuf Xs, Xsp, sigs2, ds_tmp;  // doublesided: shifted spectrum (and its perm_bin copy), its signal descriptor, second-pass rows
     int slots = 0;
     long long slot_elems = 0;
     bool two_phase = false;
@@ -310,7 +312,10 @@ int ctx_prepare(fcwt_context* ctx) {
 void plan_release(fcwt_plan* p) {
     if (p->graph) cudaGraphExecDestroy(p->graph);
     p->graph = nullptr;
-    for (auto& s : p->sig) s.X.release();
+    for (auto& s : p->sig) {
+        s.X.release();
+        s.Xp.release();
+    }
     for (auto& t : p->tables) {
         t.mother.release();
         t.tw.release();
@@ -325,7 +330,9 @@ void plan_release(fcwt_plan* p) {
     p->tc_rows.release();
     p->tc_units.release();
     p->tc_wts.release();
+    p->tc_tabs.release();
     p->Xs.release();
+    p->Xsp.release();
     p->sigs2.release();
     p->ds_tmp.release();
     p->shifted.release();
@@ -335,8 +342,6 @@ void plan_release(fcwt_plan* p) {
         if (u.done) cudaEventDestroy(u.done);
         u = fcwt_plan::UploadSlot{};
     }
-    p->tmaps.release();
-    p->graph_tmaps.release();
 }
 
 fcwt_plan* plan_new(fcwt_context* ctx) {
@@ -372,28 +377,34 @@ double queue_makespan(const std::vector<double>& cost, int ctas) {
 }
 
 // Work list of the tensor-core engine: the rows in order, with the last K
-// rows split into 2, 4 or 8 parts of their column groups when a simulation of
-// the queue says that finishes sooner. Cost model in column-group times: a
-// unit costs its groups plus about 1.2 for the per-row pre-pass and prologue.
+// rows split into 2, 4 or 8 parts of their tiles when a simulation of the
+// queue says that finishes sooner. Cost model in tile times: a unit costs its
+// tiles plus kUnitOverhead for what its first tile waits for. Only the tail of a
+// long list is simulated (two to three rounds of rows of one length before it
+// end at about the same time on every CTA): the simulation of all 8192 rows of a
+// training plan took longer than the transform.
 std::vector<int> plan_tc_units(const std::vector<int>& tc_rows, const std::vector<int>& groups, int ctas) {
-    constexpr double kUnitOverhead = 1.2;
+    constexpr double kUnitOverhead = 0.4;
     const int n = (int)tc_rows.size();
-    std::vector<int> best;
-    for (int g : tc_rows) best.push_back(g);
+    std::vector<int> best = tc_rows;
     if (n == 0 || ctas <= 1) return best;
+    const int n0 = n > 3 * ctas ? (n - 2 * ctas) / ctas * ctas : 0;  // rows before the tail
     std::vector<double> cost;
-    for (int i = 0; i < n; i++) cost.push_back(kUnitOverhead + groups[(size_t)i]);
+    for (int i = n0; i < n; i++) cost.push_back(kUnitOverhead + groups[(size_t)i]);
     double best_t = queue_makespan(cost, ctas);
+    std::vector<int> tail;
     for (int lp = 1; lp <= 3; lp++) {
         const int parts = 1 << lp;
+        int lastK = 0;
         for (int K : {ctas / 8, ctas / 4, ctas / 2, ctas, 2 * ctas}) {
-            K = std::min(K, n);
-            if (K <= 0) continue;
+            K = std::min(K, n - n0);
+            if (K <= lastK) continue;
+            lastK = K;
             std::vector<int> units;
             cost.clear();
-            for (int i = 0; i < n; i++) {
+            for (int i = n0; i < n; i++) {
                 const int ng = groups[(size_t)i];
-                if (i < n - K || ng < 2 * parts) {
+                if (i < n - K || ng < parts) {
                     units.push_back(tc_rows[(size_t)i]);
                     cost.push_back(kUnitOverhead + ng);
                     continue;
@@ -401,7 +412,7 @@ std::vector<int> plan_tc_units(const std::vector<int>& tc_rows, const std::vecto
                 for (int part = 0; part < parts; part++) {
                     const int e = fcwt::tc_unit(tc_rows[(size_t)i], lp, part);
                     int gb, ge;
-                    fcwt::tc_unit_groups(e, ng, &gb, &ge);
+                    fcwt::tc_unit_tiles(e, ng, &gb, &ge);
                     if (ge <= gb) continue;
                     units.push_back(e);
                     cost.push_back(kUnitOverhead + (ge - gb));
@@ -410,9 +421,13 @@ std::vector<int> plan_tc_units(const std::vector<int>& tc_rows, const std::vecto
             const double t = queue_makespan(cost, ctas);
             if (t < best_t * 0.995) {
                 best_t = t;
-                best = units;
+                tail = units;
             }
         }
+    }
+    if (!tail.empty()) {
+        best.resize((size_t)n0);
+        best.insert(best.end(), tail.begin(), tail.end());
     }
     return best;
 }
@@ -446,6 +461,8 @@ int plan_build(fcwt_plan* P) {
     long long tc_wts_elems = 0;       // size of their weight table
     std::vector<int> wts_rows;        // rows that own a weight-table entry
     std::map<std::array<uint32_t, 12>, long long> wts_owner;
+    std::map<std::array<int, 3>, long long> tabs;  // (log2 columns, kp, log2R) -> offset of the operand tables
+    long long tabs_bytes = 0;
     std::vector<Item> items;
     std::vector<int> compat_rows;     // compat_align: shifted rows (descriptor indices)
     int max_two_phase_log2N = 0;
@@ -462,6 +479,19 @@ int plan_build(fcwt_plan* P) {
             return fail(FCWT_ERR_UNSUPPORTED, "time decimation " + std::to_string(S.dec) + " needs N >= 8192 x " +
                                                   std::to_string(S.dec) + " for a padded length above 8192 (N = " +
                                                   std::to_string(sp.N) + ")");
+        // tensor-core engine: R = 16, or 8 for decimated lengths N' <= 16384 whose windows fit
+        S.log2R = 0;
+        const bool tc_on = ctx->engine_mode == FCWT_ENGINE_TENSOR_CORES ||
+                           (ctx->engine_mode == FCWT_ENGINE_AUTO && ctx->tune[sp.log2N].engine == 0);
+        if (tc_on && sp.N >= kTcMinN && Mfull / S.dec >= kGroupCols) {
+            const int Np = sp.N / S.dec;
+            S.log2R = Np > kTcMinN ? 4 : 3;
+            if (Np == kTcMinN)
+                for (int r = S.rb; r < S.re; r += S.rstride) {
+                    const RowPlan& rp = sp.rows[(size_t)r];
+                    if (rp.hi - (rp.lo / 128) * 128 > kTcMaxKc * 128) S.log2R = 4;
+                }
+        }
         for (int r = S.rb; r < S.re; r += S.rstride) {
             const RowPlan& rp = sp.rows[(size_t)r];
             const int ro = (r - S.rb) / S.rstride;  // output row
@@ -496,18 +526,33 @@ int plan_build(fcwt_plan* P) {
             d.kp = 0;
             d.imag = P->imag ? 1 : 0;
             const int g = (int)rows.size();
-            // tensor-core rows: window [L, L + 1024 kp), L a multiple of 1024, kp <= 16
+            // tensor-core rows: the window fits kTcMaxKc blocks of P2 bins, or folds onto them
+            // (decimated rows whose padded length N / dec is kTcMaxKc P2)
             int tc_kp = 0;
-            const bool tc_on = ctx->engine_mode == FCWT_ENGINE_TENSOR_CORES ||
-                               (ctx->engine_mode == FCWT_ENGINE_AUTO && ctx->tune[sp.log2N].engine == 0);
-            if (tc_on && sp.N >= kTcMinN && Mfull / S.dec >= kGroupCols) {
-                const int L = rp.hi > rp.lo ? (rp.lo / kP2) * kP2 : 0;
-                const int kw = rp.hi > rp.lo ? (rp.hi - L + kP2 - 1) / kP2 : 0;
-                if (kw <= kTcMaxKp) tc_kp = kw <= 8 ? 8 : 16;
-                if (tc_kp) d.L = L;
+            if (S.log2R) {
+                const int P2 = 16 << S.log2R;
+                const int L = rp.hi > rp.lo ? (rp.lo / P2) * P2 : 0;
+                const int kw = rp.hi > rp.lo ? (rp.hi - L + P2 - 1) / P2 : 0;
+                const bool folded = kw > kTcMaxKc && sp.N / S.dec == kTcMaxKc * P2;
+                if (kw <= kTcMaxKc || folded) {
+                    tc_kp = kw <= 16 ? 16 : kw <= 32 ? 32 : kTcMaxKc;
+                    d.L = L;
+                    d.log2R = S.log2R;
+                    d.folds = folded ? (kw + kTcMaxKc - 1) / kTcMaxKc : 1;
+                }
             }
             d.kp = tc_kp;
             d.woff = 0;
+            if (tc_kp) {
+                int log2M = -4 - d.log2R;
+                for (int v = sp.N / S.dec; v > 1; v >>= 1) log2M++;
+                auto it = tabs.find({log2M, tc_kp, d.log2R});
+                if (it == tabs.end()) {
+                    it = tabs.emplace(std::array<int, 3>{log2M, tc_kp, d.log2R}, tabs_bytes).first;
+                    tabs_bytes += (long long)tc_table_bytes() * tc_table_blocks(log2M);
+                }
+                d.aoff = it->second;
+            }
             if (tc_kp) {
                 // rows whose weights are the same function of q share one table entry
                 // (e.g. many channels on one grid); rows with stale bins never do
@@ -516,7 +561,7 @@ int plan_build(fcwt_plan* P) {
                 if (d.stale < 0) {
                     const float fk[6] = {d.step, d.ca, d.cb, d.cnorm, d.out_scale, 0.0f};
                     key = {(uint32_t)sp.log2N, (uint32_t)d.mode, (uint32_t)d.L, (uint32_t)d.lo, (uint32_t)d.hi,
-                           (uint32_t)d.proc, (uint32_t)d.kp, 0, 0, 0, 0, 0};
+                           (uint32_t)d.proc, (uint32_t)(d.kp | d.log2R << 8 | d.folds << 12), 0, 0, 0, 0, 0};
                     for (int k = 0; k < 5; k++) std::memcpy(&key[7 + k], &fk[k], 4);
                     auto it = wts_owner.find(key);
                     if (it != wts_owner.end()) {
@@ -526,7 +571,7 @@ int plan_build(fcwt_plan* P) {
                 }
                 if (!shared) {
                     d.woff = tc_wts_elems;
-                    tc_wts_elems += (long long)kP2 * tc_kp;
+                    tc_wts_elems += (long long)(16 << d.log2R) * tc_kp * d.folds;
                     if (d.stale < 0) wts_owner.emplace(key, d.woff);
                     wts_rows.push_back((int)rows.size());
                 }
@@ -600,6 +645,8 @@ int plan_build(fcwt_plan* P) {
         PlanSignal& S = P->sig[(size_t)s];
         FCWT_CUDA_TRY(S.X.ensure((size_t)S.sp.N * sizeof(float2)));
         sds[(size_t)s].X = S.X.as<float2>();
+        if (S.log2R) FCWT_CUDA_TRY(S.Xp.ensure((size_t)(S.sp.N / 2) * sizeof(float2)));
+        sds[(size_t)s].Xp = S.log2R ? S.Xp.as<float2>() : nullptr;
         sds[(size_t)s].mother = P->tables[(size_t)S.table].mother.as<float>();
         sds[(size_t)s].tw = P->tables[(size_t)S.table].tw.as<float2>();
         sds[(size_t)s].log2N = S.sp.log2N;
@@ -609,7 +656,6 @@ int plan_build(fcwt_plan* P) {
     if (nsig > 1) {
         FCWT_CUDA_TRY(P->fwd_tmp.ensure(tmp_elems * sizeof(float2)));
         FCWT_CUDA_TRY(P->fwd_jobs.ensure((size_t)nsig * sizeof(FwdJob)));
-        FCWT_CUDA_TRY(P->tmaps.ensure((size_t)nsig * sizeof(CUtensorMap)));
     }
     FCWT_CUDA_TRY(P->pool.ensure(std::max<size_t>(pool.size(), 1) * sizeof(float)));
     FCWT_CUDA_TRY(P->sigs.ensure(sds.size() * sizeof(SigDesc)));
@@ -626,16 +672,26 @@ int plan_build(fcwt_plan* P) {
         FCWT_CUDA_TRY(P->tc_rows.ensure(tc_rows.size() * sizeof(int)));
         FCWT_CUDA_TRY(cudaMemcpyAsync(P->tc_rows.p, tc_rows.data(), tc_rows.size() * sizeof(int),
                                       cudaMemcpyHostToDevice, st));
-        std::vector<int> groups;
-        for (int g : tc_rows) {
-            const RowDesc& d = rows[(size_t)g];
-            groups.push_back((1 << (P->sig[(size_t)d.sig].sp.log2N - kLog2P2)) / d.dec / kGroupCols);
+        std::vector<int> units;
+        for (int k = 0; k < 2; k++) {
+            std::vector<int> sel, tiles;
+            for (int g : tc_rows) {
+                const RowDesc& d = rows[(size_t)g];
+                if (d.log2R != 4 - k) continue;
+                sel.push_back(g);
+                tiles.push_back(std::max(1, (P->sig[(size_t)d.sig].sp.N / d.dec) >> (11 + d.log2R)));
+            }
+            const std::vector<int> u = plan_tc_units(sel, tiles, ctx->num_sms);
+            P->n_units[k] = (int)u.size();
+            units.insert(units.end(), u.begin(), u.end());
         }
-        const std::vector<int> units = plan_tc_units(tc_rows, groups, ctx->num_sms);
-        P->n_units = (int)units.size();
         FCWT_CUDA_TRY(P->tc_units.ensure(units.size() * sizeof(int)));
         FCWT_CUDA_TRY(cudaMemcpyAsync(P->tc_units.p, units.data(), units.size() * sizeof(int),
                                       cudaMemcpyHostToDevice, st));
+        FCWT_CUDA_TRY(P->tc_tabs.ensure((size_t)tabs_bytes));
+        for (const auto& T : tabs)
+            FCWT_CUDA_TRY(launch_tc_tables(T.first[0], T.first[1], T.first[2], P->tc_tabs.as<unsigned char>() + T.second,
+                                           st));
         FCWT_CUDA_TRY(P->tc_wts.ensure((size_t)tc_wts_elems * sizeof(float)));
         DevBuf owners;
         FCWT_CUDA_TRY(owners.ensure(wts_rows.size() * sizeof(int)));
@@ -657,6 +713,8 @@ int plan_build(fcwt_plan* P) {
         FCWT_CUDA_TRY(P->Xs.ensure((size_t)S.sp.N * sizeof(float2)));
         SigDesc s2 = sds[0];
         s2.X = P->Xs.as<float2>();
+        if (S.log2R) FCWT_CUDA_TRY(P->Xsp.ensure((size_t)(S.sp.N / 2) * sizeof(float2)));
+        s2.Xp = S.log2R ? P->Xsp.as<float2>() : nullptr;
         FCWT_CUDA_TRY(P->sigs2.ensure(sizeof(SigDesc)));
         FCWT_CUDA_TRY(cudaMemcpyAsync(P->sigs2.p, &s2, sizeof(SigDesc), cudaMemcpyHostToDevice, st));
         FCWT_CUDA_TRY(P->ds_tmp.ensure(std::max<size_t>((size_t)S.rows_out() * (size_t)S.n_out(), 1) * sizeof(float2)));
@@ -666,8 +724,8 @@ int plan_build(fcwt_plan* P) {
 }
 
 // Queue counters of one execution: [0] item queue; a_done[rows]; b_done[rows];
-// tensor-core row queue.
-size_t plan_counters(const fcwt_plan* P) { return 2 + 2 * (size_t)P->n_rows; }
+// two tensor-core row queues.
+size_t plan_counters(const fcwt_plan* P) { return 3 + 2 * (size_t)P->n_rows; }
 
 // (table, count) groups of the batched forward jobs, in table order.
 void job_groups(const fcwt_plan* P, std::vector<std::pair<int, int>>& groups) {
@@ -697,22 +755,6 @@ int upload_slot(fcwt_plan* P, size_t bytes, fcwt_plan::UploadSlot** out) {
     return FCWT_OK;
 }
 
-// The tensor maps of every output of a batched plan (entry s for output s)
-// and the mask of the outputs whose map could be encoded.
-void build_output_maps(const fcwt_plan* P, void* const* dout, int out_type, CUtensorMap* maps,
-                       unsigned long long* mask) {
-    for (int i = 0; i < fcwt::kMaxOuts / 64; i++) mask[i] = 0;
-    for (size_t s = 0; s < P->sig.size(); s++) {
-        const PlanSignal& S = P->sig[s];
-        std::memset(&maps[s], 0, sizeof(CUtensorMap));
-        if (S.rows_out() == 0 || S.sp.N < fcwt::kTcMinN) continue;
-        const bool ok = out_type == FCWT_OUT_C64
-                            ? encode_output_map(dout[s], S.n_out(), S.sp.M / S.dec, S.rows_out(), &maps[s])
-                            : encode_output_map16(dout[s], S.n_out(), S.sp.M / S.dec, S.rows_out(), &maps[s]);
-        if (ok) mask[s >> 6] |= 1ull << (s & 63);
-    }
-}
-
 // Fills `jobs` with the forward jobs of all signals ordered by table.
 void build_jobs(fcwt_plan* P, const void* const* din, std::vector<std::pair<int, int>>& groups, fcwt::FwdJob* jobs) {
     using namespace fcwt;
@@ -732,7 +774,8 @@ void build_jobs(fcwt_plan* P, const void* const* din, std::vector<std::pair<int,
             j.in_r = S.sp.is_complex ? nullptr : (const float*)din[s];
             j.in_c = S.sp.is_complex ? (const float2*)din[s] : nullptr;
             j.n = S.sp.n;
-            j.pad = 0;
+            j.log2R = S.log2R;
+            j.Xp = S.Xp.as<float2>();
             j.X = S.X.as<float2>();
             j.tmp = P->fwd_tmp.as<float2>() + tmp_off[(size_t)s];
         }
@@ -740,14 +783,12 @@ void build_jobs(fcwt_plan* P, const void* const* din, std::vector<std::pair<int,
     job_groups(P, groups);
 }
 
-int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type,
-                 bool graph_maps = false);
+int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type);
 int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* graph_jobs);
 
 // Enqueues the forward FFTs and the row engine for device-resident inputs and
 // outputs (no host synchronisation, so it can be captured into a graph).
-// graph_jobs: device copy of the forward jobs prepared before a capture; the
-// per-output tensor maps of a batched plan are then plan->graph_tmaps.
+// graph_jobs: device copy of the forward jobs prepared before a capture.
 int plan_enqueue(fcwt_plan* P, const void* const* din, void* const* dout, int out_type, bool allow_profiling,
                  const fcwt::FwdJob* graph_jobs = nullptr) {
     using namespace fcwt;
@@ -773,13 +814,14 @@ int plan_enqueue(fcwt_plan* P, const void* const* din, void* const* dout, int ou
         }
         FCWT_CUDA_TRY(cudaEventRecord(ev.first, st));
     }
-    rc = enqueue_rows(P, P->sigs.as<SigDesc>(), dout, out_type, graph_jobs != nullptr);
+    rc = enqueue_rows(P, P->sigs.as<SigDesc>(), dout, out_type);
     if (rc) return rc;
     if (P->doublesided) {
         // the mirrored half: exp(-2 pi i t / N) conj(V), V the rows on the shifted spectrum
         const PlanSignal& S = P->sig[0];
         const float2* tw = P->tables[(size_t)S.table].tw.as<float2>();
-        FCWT_CUDA_TRY(launch_shift_spectrum(S.X.as<float2>(), S.sp.log2N, P->Xs.as<float2>(), st));
+        FCWT_CUDA_TRY(launch_shift_spectrum(S.X.as<float2>(), S.sp.log2N, P->Xs.as<float2>(),
+                                            S.log2R ? P->Xsp.as<float2>() : nullptr, S.log2R, st));
         void* tmp_out[1] = {P->ds_tmp.p};
         rc = enqueue_rows(P, P->sigs2.as<SigDesc>(), tmp_out, out_type);
         if (rc) return rc;
@@ -819,7 +861,8 @@ int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* gr
         FCWT_CUDA_TRY(launch_forward(S.sp.is_complex ? nullptr : (const float*)din[0],
                                      S.sp.is_complex ? (const float2*)din[0] : nullptr, S.sp.n, S.sp.log2N,
                                      P->tables[(size_t)S.table].tw.as<float2>(), S.X.as<float2>(),
-                                     ctx->tmp.as<float2>(), st, &n_fwd));
+                                     ctx->tmp.as<float2>(), st, &n_fwd, S.log2R ? S.Xp.as<float2>() : nullptr,
+                                     S.log2R));
         ctx->kernel_launches += n_fwd;
     } else {
         // batched forward FFTs, one launch sequence per padded length
@@ -853,7 +896,7 @@ int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* gr
 
 // The row-engine launches of one pass over the plan's rows, reading the
 // spectra of `dsigs` and writing `dout`.
-int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type, bool graph_maps) {
+int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type) {
     using namespace fcwt;
     fcwt_context* ctx = P->ctx;
     cudaStream_t st = ctx->stream;
@@ -880,14 +923,13 @@ int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, in
     CUtensorMap omap;
     std::memset(&omap, 0, sizeof(omap));
     int map_ok = 0;
-    if (nsig == 1 && (P->two_phase || P->n_tc > 0)) {
+    if (nsig == 1 && P->two_phase) {
         const PlanSignal& S = P->sig[0];
         if (out_type == FCWT_OUT_C64)
             map_ok = encode_output_map(dout[0], S.n_out(), S.sp.M / S.dec, S.rows_out(), &omap) ? 1 : 0;
         else
             map_ok = encode_output_map16(dout[0], S.n_out(), S.sp.M / S.dec, S.rows_out(), &omap) ? 1 : 0;
     }
-    // the CUDA-core engine's two-phase rows store through the same map
     ep.tma_store = P->two_phase ? map_ok : 0;
     const int grid = std::max(1, std::min(P->n_items, ctx->engine_ctas));
     if (P->n_tc > 0) {
@@ -895,35 +937,18 @@ int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, in
         std::memset(&tp, 0, sizeof(tp));
         tp.sigs = ep.sigs;
         tp.rows = ep.rows;
-        tp.row_list = P->tc_units.as<int>();
-        tp.n_list = P->n_units;
-        tp.stale_pool = ep.stale_pool;
         tp.wts = P->tc_wts.as<float>();
-        tp.counter = ctx->counters.as<unsigned>() + n_counters - 1;
+        tp.atab = P->tc_tabs.as<unsigned char>();
         for (int s = 0; s < nsig; s++) tp.outs[s] = dout[s];
         tp.err = ep.err;
-        tp.tma_store = map_ok;
-        tp.decimated = P->sig.size() == 1 && P->sig[0].dec > 1;
-        if (nsig > 1) {
-            // one tensor map per output, in device memory
-            if (graph_maps) {
-                tp.tmaps = P->graph_tmaps.as<CUtensorMap>();
-                for (int k = 0; k < kMaxOuts / 64; k++) tp.tmap_mask[k] = P->graph_tmap_mask[(size_t)k];
-            } else {
-                fcwt_plan::UploadSlot* u = nullptr;
-                int rc = upload_slot(P, (size_t)nsig * sizeof(CUtensorMap), &u);
-                if (rc) return rc;
-                build_output_maps(P, dout, out_type, static_cast<CUtensorMap*>(u->host), tp.tmap_mask);
-                FCWT_CUDA_TRY(cudaMemcpyAsync(P->tmaps.p, u->host, (size_t)nsig * sizeof(CUtensorMap),
-                                              cudaMemcpyHostToDevice, st));
-                FCWT_CUDA_TRY(cudaEventRecord(u->done, st));
-                u->pending = true;
-                tp.tmaps = P->tmaps.as<CUtensorMap>();
-            }
-            tp.tma_store = 1;
+        for (int k = 0; k < 2; k++) {
+            if (P->n_units[k] == 0) continue;
+            tp.row_list = P->tc_units.as<int>() + (k ? P->n_units[0] : 0);
+            tp.n_list = P->n_units[k];
+            tp.counter = ctx->counters.as<unsigned>() + n_counters - 2 + k;
+            FCWT_CUDA_TRY(launch_tc(tp, 4 - k, out_type, std::max(1, std::min(P->n_units[k], ctx->num_sms)), st));
+            ctx->kernel_launches += 1;
         }
-        FCWT_CUDA_TRY(launch_tc(tp, omap, out_type, std::max(1, std::min(P->n_units, ctx->num_sms)), st));
-        ctx->kernel_launches += 1;
     }
     if (P->n_items > 0) {
         FCWT_CUDA_TRY(launch_engine(ep, omap, grid, st));
@@ -991,25 +1016,18 @@ int run_pipelined(fcwt_plan* P, const void* din, void* hout, int out_type) {
         // rows r0.. of the plan write at out_off = r * row elements: shift the base so they land in the
         // slot (an address below the slot that no access uses; only base + out_off is dereferenced)
         char* base = reinterpret_cast<char*>(reinterpret_cast<uintptr_t>(stage) - (uintptr_t)r0 * row_bytes);
-        CUtensorMap omap;
-        std::memset(&omap, 0, sizeof(omap));
-        const int map_ok = out_type == FCWT_OUT_C64
-                               ? (encode_output_map(base, S.n_out(), S.sp.M / S.dec, r1, &omap) ? 1 : 0)
-                               : (encode_output_map16(base, S.n_out(), S.sp.M / S.dec, r1, &omap) ? 1 : 0);
         TcParams tp;
         std::memset(&tp, 0, sizeof(tp));
         tp.sigs = P->sigs.as<SigDesc>();
         tp.rows = P->rows.as<RowDesc>();
         tp.row_list = P->tc_rows.as<int>() + r0;  // tc_rows lists the rows in order
         tp.n_list = r1 - r0;
-        tp.stale_pool = P->pool.as<float>();
         tp.wts = P->tc_wts.as<float>();
+        tp.atab = P->tc_tabs.as<unsigned char>();
         tp.counter = ctx->counters.as<unsigned>() + b;
         tp.outs[0] = base;
         tp.err = ctx->err.as<int>();
-        tp.tma_store = map_ok;
-        tp.decimated = P->sig.size() == 1 && P->sig[0].dec > 1;
-        FCWT_CUDA_TRY(launch_tc(tp, omap, out_type, std::max(1, std::min(r1 - r0, ctx->num_sms)), st));
+        FCWT_CUDA_TRY(launch_tc(tp, S.log2R, out_type, std::max(1, std::min(r1 - r0, ctx->num_sms)), st));
         ctx->kernel_launches += 1;
         FCWT_CUDA_TRY(cudaEventRecord(ctx->pipe_done[slot], st));
         FCWT_CUDA_TRY(cudaStreamWaitEvent(ctx->copy_stream, ctx->pipe_done[slot], 0));
@@ -1635,18 +1653,13 @@ int fcwt_plan_execute_graph(fcwt_plan* plan, const void* const* inputs, void* co
             FCWT_CUDA_TRY(ctx->scratch.ensure((size_t)plan->slots * (size_t)plan->slot_elems * sizeof(float2)));
         const fcwt::FwdJob* gj = nullptr;
         if (nsig > 1) {
-            // the graph reads its jobs and tensor maps from buffers of its own,
+            // the graph reads its jobs from a buffer of its own,
             // filled once here (synchronously, before the capture)
             std::vector<std::pair<int, int>> groups;
             std::vector<fcwt::FwdJob> jobs((size_t)nsig);
             build_jobs(plan, inputs, groups, jobs.data());
             FCWT_CUDA_TRY(plan->graph_jobs.ensure((size_t)nsig * sizeof(fcwt::FwdJob)));
             FCWT_CUDA_TRY(cudaMemcpy(plan->graph_jobs.p, jobs.data(), (size_t)nsig * sizeof(fcwt::FwdJob),
-                                     cudaMemcpyHostToDevice));
-            std::vector<CUtensorMap> maps((size_t)nsig);
-            build_output_maps(plan, outputs, out_type, maps.data(), plan->graph_tmap_mask.data());
-            FCWT_CUDA_TRY(plan->graph_tmaps.ensure((size_t)nsig * sizeof(CUtensorMap)));
-            FCWT_CUDA_TRY(cudaMemcpy(plan->graph_tmaps.p, maps.data(), (size_t)nsig * sizeof(CUtensorMap),
                                      cudaMemcpyHostToDevice));
             gj = plan->graph_jobs.as<fcwt::FwdJob>();
         }
@@ -1792,7 +1805,8 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
         j.in_r = x + (size_t)b * n;
         j.in_c = nullptr;
         j.n = n;
-        j.pad = 0;
+        j.log2R = 0;
+        j.Xp = nullptr;
         j.X = ctx->adj_x.as<float2>() + (size_t)b * N;
         j.tmp = ctx->adj_tmp.as<float2>() + (size_t)b * N;
     }
@@ -1819,7 +1833,8 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
                 j.in_r = nullptr;
                 j.in_c = G + ((size_t)b * fn + i0 + i) * n;
                 j.n = n;
-                j.pad = 0;
+                j.log2R = 0;
+        j.Xp = nullptr;
                 j.X = ctx->adj_g.as<float2>() + ((size_t)b * nr + i) * N;
                 j.tmp = ctx->adj_tmp.as<float2>() + ((size_t)b * nr + i) * N;
             }
@@ -1840,7 +1855,8 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
         j.in_r = nullptr;
         j.in_c = ctx->adj_h.as<float2>() + (size_t)b * N;
         j.n = N;
-        j.pad = 0;
+        j.log2R = 0;
+        j.Xp = nullptr;
         j.X = ctx->adj_g.as<float2>() + (size_t)b * N;
         j.tmp = ctx->adj_tmp.as<float2>() + (size_t)b * N;
     }

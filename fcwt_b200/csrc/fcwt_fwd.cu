@@ -168,7 +168,9 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
         float2 v = res[t];
         if (mode == 0 && col > 0 && k > 0)
             v = cmul(v, fft_tw<SIGN>(tw, log2T, (unsigned)(col * k) << (log2T - log2C)));
-        dst[col + (k << log2S)] = v;
+        const int o = col + (k << log2S);
+        dst[o] = v;
+        if (dst_sel == 1 && J.log2R && o < (1 << (log2C - 1))) J.Xp[perm_bin(o, J.log2R)] = v;
     }
 }
 
@@ -193,6 +195,7 @@ __global__ void k_r2c_split(const FwdJob* __restrict__ jobs, FwdJob one, int log
     const float2 xk = make_float2(E.x + wo.x, E.y + wo.y);
     const float2 yk = make_float2(E.x - wo.x, wo.y - E.y);
     X[k] = xk;
+    if (J.log2R && k < H) J.Xp[perm_bin(k, J.log2R)] = xk;
     if (k == 0) {
         X[H] = yk;
         return;
@@ -200,6 +203,7 @@ __global__ void k_r2c_split(const FwdJob* __restrict__ jobs, FwdJob one, int log
     X[N - k] = make_float2(xk.x, -xk.y);
     if (2 * k < H) {
         X[H - k] = yk;
+        if (J.log2R) J.Xp[perm_bin(H - k, J.log2R)] = yk;
         X[H + k] = make_float2(yk.x, -yk.y);
     }
 }
@@ -260,7 +264,7 @@ static cudaError_t fft_signals(const FwdJob* jobs, const FwdJob& one, int njobs,
 }
 
 cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log2N, const float2* tw,
-                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels) {
+                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R) {
     *n_kernels = 0;
     if (log2N == 0) {
         // N == 1: the DFT is the identity (one sample or none).
@@ -279,9 +283,10 @@ cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log
     one.in_r = in_r;
     one.in_c = in_r ? nullptr : in_c;
     one.n = n;
-    one.pad = 0;
+    one.log2R = Xp ? log2R : 0;
     one.X = out;
     one.tmp = tmp;
+    one.Xp = Xp;
     return fft_signals<-1>(nullptr, one, 1, log2N, tw, in_r != nullptr, st, n_kernels);
 }
 

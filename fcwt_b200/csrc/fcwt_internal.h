@@ -40,6 +40,7 @@ struct SigDesc {
     const float2* X;       // forward spectrum, >= N/2 bins
     const float* mother;   // mother table, N entries
     const float2* tw;      // [0,1024): w_N^j ; [1024, 1024+M): w_N^{1024 j}
+    const float2* Xp;      // tensor-core rows: bins < N/2 in the order of perm_bin, null without such rows
     int log2N;
     int n;
 };
@@ -65,12 +66,14 @@ struct RowDesc {
     int mode;         // 0: reference mother-table weights; 1: continuous Morlet
     float ca, cb;     // continuous Morlet: u = ca*q - cb
     float cnorm;      // continuous Morlet amplitude (the mother table's norm)
-    int kp;           // tensor-core rows: 1024-bin blocks of the window, padded to 8 or 16
-    long long woff;   // tensor-core rows: offset of the row's 1024*kp weights in the plan's table
+    int kp;           // tensor-core rows: blocks of P2 = 16 << log2R bins in the window (16, 32 or 64)
+    int log2R;        // tensor-core rows: 4, or 3 (see fcwt_tc.cu)
+    int folds;        // tensor-core rows: windows of kp blocks folded onto each other (decimated rows)
+    long long woff;   // tensor-core rows: offset of the row's P2*kp*folds weights in the plan's table
+    long long aoff;   // tensor-core rows: byte offset of the row's operand tables (columns N'/P2, kp)
     int imag;         // 1: wavelet with imag_frequency, every product multiplied by i
     int dec;          // time decimation D (power of two): output sample t' is y[D t']
     int n_out;        // output samples of the row: ceil(n / D)
-    int pad_;
 };
 
 enum ItemType : int { ITEM_FUSED = 0, ITEM_PHASE1 = 1, ITEM_PHASE2 = 2, ITEM_SMALL = 3, ITEM_PHASE1W = 4 };
@@ -94,10 +97,19 @@ struct FwdJob {
     const float* in_r;
     const float2* in_c;
     int n;
-    int pad;
+    int log2R;   // forward transforms: also write bins < N/2 to Xp in the order of perm_bin (0: don't)
     float2* X;
     float2* tmp;
+    float2* Xp;
 };
+
+// Position of bin q in the permuted spectrum copy: within its block of P2 = 16 R
+// bins, bin kl + 16 kb sits at kl R + kb (the accumulator order of fcwt_tc.cu).
+__host__ __device__ inline int perm_bin(int q, int log2R) {
+    const int P2 = 16 << log2R;
+    const int k2 = q & (P2 - 1);
+    return (q - k2) + ((k2 & 15) << log2R) + (k2 >> 4);
+}
 
 // Everything the row engine needs for one launch.
 struct EngineParams {
@@ -116,33 +128,27 @@ struct EngineParams {
     int tma_store;             // phase-2 outputs via the tensor map (buffer 0, complex64, even n)
 };
 
-// Tensor-core row engine (fcwt_tc.cu): rows whose window [L, L + 1024 kp)
-// (L a multiple of 1024) spans at most kTcMaxKp blocks, for N >= kTcMinN.
-constexpr int kTcMaxKp = 16;
+// Tensor-core row engine (fcwt_tc.cu): rows whose window [L, L + kTcMaxKc P2)
+// (L a multiple of P2) holds all nonzero bins, for N >= kTcMinN.
+constexpr int kTcMaxKc = 64;
 constexpr int kTcMinN = 16384;
 
 // Entries of the tensor-core engine's work list: a row index, or one of 2, 4
-// or 8 parts of a row's column groups (the last entries of a launch, so that
+// or 8 parts of a row's 128-column tiles (the last entries of a launch, so that
 // its final wave is finer than whole rows): row | log2(parts) << 24 | part << 26.
 constexpr int kUnitRowBits = 24;
 constexpr int kUnitRowMask = (1 << kUnitRowBits) - 1;
 __host__ __device__ constexpr int tc_unit(int row, int log2parts, int part) {
     return row | (log2parts << kUnitRowBits) | (part << (kUnitRowBits + 2));
 }
-// Column groups [gb, ge) of a unit of a row with ng groups; part ranges hold an
-// even number of groups so that the two halves of a CTA share them evenly.
-__host__ __device__ inline void tc_unit_groups(int entry, int ng, int* gb, int* ge) {
+// Tiles [sb, se) of a unit of a row with nt tiles.
+__host__ __device__ inline void tc_unit_tiles(int entry, int nt, int* sb, int* se) {
     const int lp = (entry >> kUnitRowBits) & 3;
     const int part = (entry >> (kUnitRowBits + 2)) & 7;
-    if (lp == 0) {
-        *gb = 0;
-        *ge = ng;
-        return;
-    }
     const int parts = 1 << lp;
-    const int chunk = (((ng + parts - 1) / parts) + 1) & ~1;
-    *gb = part * chunk < ng ? part * chunk : ng;
-    *ge = *gb + chunk < ng ? *gb + chunk : ng;
+    const int chunk = (nt + parts - 1) / parts;
+    *sb = part * chunk < nt ? part * chunk : nt;
+    *se = *sb + chunk < nt ? *sb + chunk : nt;
 }
 
 struct TcParams {
@@ -150,17 +156,11 @@ struct TcParams {
     const RowDesc* rows;
     const int* row_list;       // work units of this launch (tc_unit entries), in queue order
     int n_list;
-    const float* stale_pool;
-    const float* wts;          // per-row daughter weights x out_scale on [L, L + 1024 kp)
+    const float* wts;          // per-row daughter weights x out_scale on the row's window
+    const unsigned char* atab;  // operand tables (RowDesc::aoff)
     unsigned* counter;         // row queue head
     void* outs[kMaxOuts];
     int* err;
-    int tma_store;             // outputs via the tensor map (buffer 0, complex64, even n)
-    int decimated;             // some row has RowDesc::dec > 1 (selects the decimating kernel)
-    // many outputs (batched plans): one tensor map per output buffer in global
-    // memory, used where bit `out_buf` of tmap_mask is set
-    const CUtensorMap* tmaps;
-    unsigned long long tmap_mask[kMaxOuts / 64];
 };
 
 // Error bits written by device code into EngineParams::err.

@@ -670,7 +670,8 @@ cudaError_t launch_twiddle(int log2N, float2* tw, cudaStream_t st) {
 // ordinary single-sided row of the same weights on the shifted spectrum
 //     J[q] = Ihat[q + 1] (q < N/2 - 1),  J[N/2 - 1] = conj(Ihat[N/2]).
 namespace dev {
-__global__ void k_shift_spectrum(const float2* __restrict__ X, int N, float2* __restrict__ J) {
+__global__ void k_shift_spectrum(const float2* __restrict__ X, int N, float2* __restrict__ J,
+                                 float2* __restrict__ Jp, int log2R) {
     const int half = N >> 1;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
         float2 v = make_float2(0.0f, 0.0f);
@@ -679,6 +680,7 @@ __global__ void k_shift_spectrum(const float2* __restrict__ X, int N, float2* __
         else if (q + 1 == half)
             v = make_float2(X[half].x, -X[half].y);
         J[q] = v;
+        if (Jp && q < half) Jp[perm_bin(q, log2R)] = v;
     }
 }
 
@@ -745,9 +747,9 @@ cudaError_t launch_align_spill(const SigDesc* sigs, const RowDesc* rows, const i
     return cudaGetLastError();
 }
 
-cudaError_t launch_shift_spectrum(const float2* X, int log2N, float2* J, cudaStream_t st) {
+cudaError_t launch_shift_spectrum(const float2* X, int log2N, float2* J, float2* Jp, int log2R, cudaStream_t st) {
     const int N = 1 << log2N;
-    dev::k_shift_spectrum<<<std::max(1, std::min(1184, (N + 255) / 256)), 256, 0, st>>>(X, N, J);
+    dev::k_shift_spectrum<<<std::max(1, std::min(1184, (N + 255) / 256)), 256, 0, st>>>(X, N, J, Jp, log2R);
     return cudaGetLastError();
 }
 

@@ -42,7 +42,7 @@ namespace fcwt {
 cudaError_t launch_mother(float fb, int N, float norm, float* out, cudaStream_t st);
 cudaError_t launch_twiddle(int log2N, float2* tw, cudaStream_t st);
 cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log2N, const float2* tw,
-                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels);
+                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R);
 cudaError_t engine_configure();
 cudaError_t engine_blocks_per_sm(int* out);
 cudaError_t launch_engine(const EngineParams& p, int grid, cudaStream_t st);
@@ -80,7 +80,7 @@ constexpr size_t kNoAllocScratchBytes = align256(kOffScratch + sizeof(float2) * 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 // ---- descriptor delivery by kernel parameters (at most 32764 bytes each)
-constexpr int kRowsPerCopy = 232;    // RowDesc per launch (232 x 120 B)
+constexpr int kRowsPerCopy = 232;    // RowDesc per launch (232 x 136 B)
 constexpr int kFloatsPerCopy = 7680; // 30 KB of stale-bin table entries
 
 struct RowCopy {
@@ -278,6 +278,7 @@ extern "C" int fcwt_cwt_noalloc(const float* input, int n, float fb, const float
         c.sig.X = X;
         c.sig.mother = mother;
         c.sig.tw = tw;
+        c.sig.Xp = nullptr;
         c.sig.log2N = sp.log2N;
         c.sig.n = n;
         for (int r0 = 0; r0 < fn; r0 += kRowsPerCopy) {
@@ -310,7 +311,7 @@ extern "C" int fcwt_cwt_noalloc(const float* input, int n, float fb, const float
     NA_TRY(launch_mother(fb, N, host::mother_norm(), mother, st));
     NA_TRY(launch_twiddle(sp.log2N, tw, st));
     int n_fwd = 0;
-    NA_TRY(launch_forward(input, nullptr, n, sp.log2N, tw, X, tmp, st, &n_fwd));
+    NA_TRY(launch_forward(input, nullptr, n, sp.log2N, tw, X, tmp, st, &n_fwd, nullptr, 0));
     EngineParams ep;
     std::memset(&ep, 0, sizeof(ep));
     ep.sigs = dsig;

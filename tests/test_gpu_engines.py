@@ -261,3 +261,37 @@ def test_maximum_padded_length(fcwt, oracle, ctx, mode):
     p.execute(x, out)
     p.close()
     assert rel_l2(out, oracle.cwt_fp64(x, sc, 2.0, 1, True)) < TOL
+
+
+# sizes where the tensor-core engine's tiling changes: one 128-column tile with
+# P2 = 128 (N = 16384), one, two, four and eight tiles with P2 = 256 (N = 32768 ..
+# 262144), n at either end of the padded length, odd and even; bands that take
+# 16, 32 and 64 blocks of the window, and decimated rows with half a tile, folded
+# windows and P2 = 256 on half a tile
+TC_EDGES = [
+    (8193, 1, 0.2), (16383, 1, 0.45), (16385, 1, 0.02), (32768, 1, 0.2), (32769, 1, 0.1), (65535, 1, 0.12),
+    (65537, 1, 0.01), (65540, 1, 0.03), (131071, 1, 0.06), (131073, 1, 0.05), (262144, 1, 0.004),
+    (16384, 2, 0.3), (32768, 2, 0.05), (65536, 4, 0.11), (65537, 8, 0.1), (100000, 16, 0.1), (99999, 4, 0.06),
+]
+
+
+@pytest.mark.parametrize("n,dec,f1", TC_EDGES)
+def test_tensor_core_tiling_edges(fcwt, oracle, n, dec, f1):
+    """Every row against the float64 oracle. Bound: split-FP16 products 2^-21
+    per element, at most 8 + 16 FP32 accumulations and 24 FP32 butterfly steps
+    of 2^-24 each: 2^-21 + 48 x 2^-24 = 3.3e-6 if all were to add up."""
+    import torch
+
+    fn = 9
+    sc = fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LOGSCALES, 100000, 60.0 * 100000 / n, 100000.0 * f1, fn)
+    x = np.random.default_rng(n + dec).standard_normal(n).astype(np.float32)
+    plan = fcwt.Plan(n, sc, fb=2.0, time_stride=dec)
+    # (the reused bins of a coarse grid widen some rows' windows past the engine's limit)
+    assert plan.stats()["tensor_core_rows"] >= 1
+    out = torch.full(plan.out_shape, float("nan"), dtype=torch.complex64, device="cuda")
+    plan.execute(torch.from_numpy(x).cuda(), out)
+    got = out.cpu().numpy()
+    plan.close()
+    ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)[:, ::dec]
+    for r in range(fn):
+        assert rel_l2(got[r], ref[r]) <= 3.3e-6, r
