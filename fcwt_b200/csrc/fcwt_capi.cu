@@ -81,6 +81,13 @@ int fail(int code, const std::string& msg) {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool own = true;  // false: a part of another buffer
+    void part_of(void* base, size_t b) {
+        release();
+        p = base;
+        bytes = b;
+        own = false;
+    }
     cudaError_t ensure(size_t b) {
         if (b <= bytes && p) return cudaSuccess;
         release();
@@ -95,9 +102,10 @@ struct DevBuf {
         return cudaSuccess;
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p && own) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        own = true;
     }
     template <class T>
     T* as() const {
@@ -228,6 +236,19 @@ struct fcwt_context {
     // host-output pipeline: copy stream, per-slot "rows done" / "block copied" events
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t pipe_done[2] = {nullptr, nullptr}, pipe_copied[2] = {nullptr, nullptr};
+    // Uploads of batched plans (forward jobs per execution) go through a ring of
+    // pinned host slots; a slot is rewritten only after the copy that read it has
+    // run (its event), so back-to-back executions never see each other's data. The
+    // ring belongs to the context: a training loop makes a plan per step, and pinning
+    // memory for each took longer than building it.
+    struct UploadSlot {
+        void* host = nullptr;
+        size_t bytes = 0;
+        cudaEvent_t done = nullptr;
+        bool pending = false;
+    };
+    std::array<UploadSlot, 4> uploads;
+    int upload_next = 0;
     // profiling
     bool profiling = false;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_used, ev_free;
@@ -269,17 +290,7 @@ struct fcwt_plan {
     DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, tc_wts, tc_tabs;
     DevBuf tc_units;  // work list of the tensor-core engine (rows, the last ones possibly split)
     int n_units[2] = {0, 0};  // units of R = 16 and, after them, of R = 8
-    // Per-execution uploads of batched plans (forward jobs) go through a ring of pinned host slots; a slot is rewritten only
-    // after the copy that read it has run (its event), so back-to-back
-    // executions with different buffers never see each other's data.
-    struct UploadSlot {
-        void* host = nullptr;
-        size_t bytes = 0;
-        cudaEvent_t done = nullptr;
-        bool pending = false;
-    };
-    std::array<UploadSlot, 4> uploads;
-    int upload_next = 0;
+    DevBuf mem;  // one allocation that holds the buffers plan_build fills
     int n_items = 0;
     int n_rows = 0;
     int n_tc = 0;  // rows run by the tensor-core engine
@@ -336,12 +347,7 @@ void plan_release(fcwt_plan* p) {
     p->sigs2.release();
     p->ds_tmp.release();
     p->shifted.release();
-    for (auto& u : p->uploads) {
-        if (u.pending && u.done) cudaEventSynchronize(u.done);
-        if (u.host) cudaFreeHost(u.host);
-        if (u.done) cudaEventDestroy(u.done);
-        u = fcwt_plan::UploadSlot{};
-    }
+    p->mem.release();
 }
 
 fcwt_plan* plan_new(fcwt_context* ctx) {
@@ -626,12 +632,94 @@ int plan_build(fcwt_plan* P) {
     P->n_items = (int)items.size();
     P->n_tc = (int)tc_rows.size();
 
-    // device buffers and tables
+    P->n_shifted = (int)compat_rows.size();
+    std::vector<int> units;
+    for (int k = 0; k < 2; k++) {
+        std::vector<int> sel, tiles;
+        for (int g : tc_rows) {
+            const RowDesc& d = rows[(size_t)g];
+            if (d.log2R != 4 - k) continue;
+            sel.push_back(g);
+            tiles.push_back(std::max(1, (P->sig[(size_t)d.sig].sp.N / d.dec) >> (11 + d.log2R)));
+        }
+        const std::vector<int> u = plan_tc_units(sel, tiles, ctx->num_sms);
+        P->n_units[k] = (int)u.size();
+        units.insert(units.end(), u.begin(), u.end());
+    }
+
+    // One device allocation for all buffers of the plan: first what the host fills
+    // (one copy), then what kernels fill. (An allocation per buffer, 136 of them for
+    // 64 signals, took 6 ms of a training step.)
+    std::vector<SigDesc> sds((size_t)nsig);
+    SigDesc sd2;
+    DevBuf owners;
+    std::vector<std::pair<DevBuf*, size_t>> want;
+    want.push_back({&P->pool, pool.size() * sizeof(float)});
+    want.push_back({&P->sigs, sds.size() * sizeof(SigDesc)});
+    want.push_back({&P->rows, rows.size() * sizeof(RowDesc)});
+    want.push_back({&P->items, items.size() * sizeof(Item)});
+    want.push_back({&P->tc_rows, tc_rows.size() * sizeof(int)});
+    want.push_back({&P->tc_units, units.size() * sizeof(int)});
+    want.push_back({&owners, wts_rows.size() * sizeof(int)});
+    want.push_back({&P->shifted, compat_rows.size() * sizeof(int)});
+    want.push_back({&P->sigs2, P->doublesided ? sizeof(SigDesc) : 0});
+    const size_t n_filled = want.size();
+    size_t tmp_elems = 0;
+    for (auto& T : P->tables) {
+        const size_t N = (size_t)1 << T.log2N;
+        want.push_back({&T.mother, N * sizeof(float)});
+        want.push_back({&T.tw, (1024 + std::max<size_t>(N / kP2, 1)) * sizeof(float2)});
+    }
+    for (auto& S : P->sig) {
+        want.push_back({&S.X, (size_t)S.sp.N * sizeof(float2)});
+        if (S.log2R) want.push_back({&S.Xp, (size_t)(S.sp.N / 2) * sizeof(float2)});
+        tmp_elems += (size_t)S.sp.N;
+    }
+    if (nsig > 1) {
+        want.push_back({&P->fwd_tmp, tmp_elems * sizeof(float2)});
+        want.push_back({&P->fwd_jobs, (size_t)nsig * sizeof(FwdJob)});
+    }
+    want.push_back({&P->tc_tabs, (size_t)tabs_bytes});
+    want.push_back({&P->tc_wts, (size_t)tc_wts_elems * sizeof(float)});
+    if (P->doublesided) {
+        const PlanSignal& S = P->sig[0];
+        want.push_back({&P->Xs, (size_t)S.sp.N * sizeof(float2)});
+        if (S.log2R) want.push_back({&P->Xsp, (size_t)(S.sp.N / 2) * sizeof(float2)});
+        want.push_back({&P->ds_tmp, (size_t)S.rows_out() * (size_t)S.n_out() * sizeof(float2)});
+    }
+    auto padded = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    size_t total = 0, filled = 0;
+    for (size_t i = 0; i < want.size(); i++) {
+        total += padded(want[i].second);
+        if (i + 1 == n_filled) filled = total;
+    }
+    FCWT_CUDA_TRY(P->mem.ensure(total));
+    size_t off = 0;
+    for (auto& w : want) {
+        w.first->part_of(P->mem.as<char>() + off, w.second);
+        off += padded(w.second);
+    }
+    for (int s = 0; s < nsig; s++) {
+        PlanSignal& S = P->sig[(size_t)s];
+        sds[(size_t)s].X = S.X.as<float2>();
+        sds[(size_t)s].Xp = S.log2R ? S.Xp.as<float2>() : nullptr;
+        sds[(size_t)s].mother = P->tables[(size_t)S.table].mother.as<float>();
+        sds[(size_t)s].tw = P->tables[(size_t)S.table].tw.as<float2>();
+        sds[(size_t)s].log2N = S.sp.log2N;
+        sds[(size_t)s].n = S.sp.n;
+    }
+    sd2 = sds[0];
+    sd2.X = P->Xs.as<float2>();
+    sd2.Xp = P->sig[0].log2R ? P->Xsp.as<float2>() : nullptr;
+    const void* src[] = {pool.data(),  sds.data(),      rows.data(),        items.data(), tc_rows.data(),
+                         units.data(), wts_rows.data(), compat_rows.data(), &sd2};
+    std::vector<char> image(filled);
+    for (size_t i = 0; i < n_filled; i++)
+        if (want[i].second)
+            std::memcpy(image.data() + (want[i].first->as<char>() - P->mem.as<char>()), src[i], want[i].second);
+    FCWT_CUDA_TRY(cudaMemcpyAsync(P->mem.p, image.data(), filled, cudaMemcpyHostToDevice, st));
     for (auto& T : P->tables) {
         const int N = 1 << T.log2N;
-        const int M = N >= kP2 ? N / kP2 : 1;
-        FCWT_CUDA_TRY(T.mother.ensure((size_t)N * sizeof(float)));
-        FCWT_CUDA_TRY(T.tw.ensure((size_t)(1024 + M) * sizeof(float2)));
         if (!P->custom_mother.empty() && (int)P->custom_mother.size() == N)
             FCWT_CUDA_TRY(cudaMemcpyAsync(T.mother.p, P->custom_mother.data(), (size_t)N * sizeof(float),
                                           cudaMemcpyHostToDevice, st));
@@ -639,86 +727,11 @@ int plan_build(fcwt_plan* P) {
             FCWT_CUDA_TRY(launch_mother(P->fb, N, host::mother_norm(), T.mother.as<float>(), st));
         FCWT_CUDA_TRY(launch_twiddle(T.log2N, T.tw.as<float2>(), st));
     }
-    std::vector<SigDesc> sds((size_t)nsig);
-    size_t tmp_elems = 0;
-    for (int s = 0; s < nsig; s++) {
-        PlanSignal& S = P->sig[(size_t)s];
-        FCWT_CUDA_TRY(S.X.ensure((size_t)S.sp.N * sizeof(float2)));
-        sds[(size_t)s].X = S.X.as<float2>();
-        if (S.log2R) FCWT_CUDA_TRY(S.Xp.ensure((size_t)(S.sp.N / 2) * sizeof(float2)));
-        sds[(size_t)s].Xp = S.log2R ? S.Xp.as<float2>() : nullptr;
-        sds[(size_t)s].mother = P->tables[(size_t)S.table].mother.as<float>();
-        sds[(size_t)s].tw = P->tables[(size_t)S.table].tw.as<float2>();
-        sds[(size_t)s].log2N = S.sp.log2N;
-        sds[(size_t)s].n = S.sp.n;
-        tmp_elems += (size_t)S.sp.N;
-    }
-    if (nsig > 1) {
-        FCWT_CUDA_TRY(P->fwd_tmp.ensure(tmp_elems * sizeof(float2)));
-        FCWT_CUDA_TRY(P->fwd_jobs.ensure((size_t)nsig * sizeof(FwdJob)));
-    }
-    FCWT_CUDA_TRY(P->pool.ensure(std::max<size_t>(pool.size(), 1) * sizeof(float)));
-    FCWT_CUDA_TRY(P->sigs.ensure(sds.size() * sizeof(SigDesc)));
-    FCWT_CUDA_TRY(P->rows.ensure(std::max<size_t>(rows.size(), 1) * sizeof(RowDesc)));
-    FCWT_CUDA_TRY(P->items.ensure(std::max<size_t>(items.size(), 1) * sizeof(Item)));
-    if (!pool.empty())
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->pool.p, pool.data(), pool.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    FCWT_CUDA_TRY(cudaMemcpyAsync(P->sigs.p, sds.data(), sds.size() * sizeof(SigDesc), cudaMemcpyHostToDevice, st));
-    if (!rows.empty())
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->rows.p, rows.data(), rows.size() * sizeof(RowDesc), cudaMemcpyHostToDevice, st));
-    if (!items.empty())
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->items.p, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice, st));
-    if (!tc_rows.empty()) {
-        FCWT_CUDA_TRY(P->tc_rows.ensure(tc_rows.size() * sizeof(int)));
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->tc_rows.p, tc_rows.data(), tc_rows.size() * sizeof(int),
-                                      cudaMemcpyHostToDevice, st));
-        std::vector<int> units;
-        for (int k = 0; k < 2; k++) {
-            std::vector<int> sel, tiles;
-            for (int g : tc_rows) {
-                const RowDesc& d = rows[(size_t)g];
-                if (d.log2R != 4 - k) continue;
-                sel.push_back(g);
-                tiles.push_back(std::max(1, (P->sig[(size_t)d.sig].sp.N / d.dec) >> (11 + d.log2R)));
-            }
-            const std::vector<int> u = plan_tc_units(sel, tiles, ctx->num_sms);
-            P->n_units[k] = (int)u.size();
-            units.insert(units.end(), u.begin(), u.end());
-        }
-        FCWT_CUDA_TRY(P->tc_units.ensure(units.size() * sizeof(int)));
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->tc_units.p, units.data(), units.size() * sizeof(int),
-                                      cudaMemcpyHostToDevice, st));
-        FCWT_CUDA_TRY(P->tc_tabs.ensure((size_t)tabs_bytes));
-        for (const auto& T : tabs)
-            FCWT_CUDA_TRY(launch_tc_tables(T.first[0], T.first[1], T.first[2], P->tc_tabs.as<unsigned char>() + T.second,
-                                           st));
-        FCWT_CUDA_TRY(P->tc_wts.ensure((size_t)tc_wts_elems * sizeof(float)));
-        DevBuf owners;
-        FCWT_CUDA_TRY(owners.ensure(wts_rows.size() * sizeof(int)));
-        FCWT_CUDA_TRY(cudaMemcpyAsync(owners.p, wts_rows.data(), wts_rows.size() * sizeof(int),
-                                      cudaMemcpyHostToDevice, st));
-        FCWT_CUDA_TRY(launch_tc_weights(P->sigs.as<SigDesc>(), P->rows.as<RowDesc>(), owners.as<int>(),
-                                        (int)wts_rows.size(), P->pool.as<float>(), P->tc_wts.as<float>(), st));
-        FCWT_CUDA_TRY(cudaStreamSynchronize(st));
-        owners.release();
-    }
-    if (!compat_rows.empty()) {
-        FCWT_CUDA_TRY(P->shifted.ensure(compat_rows.size() * sizeof(int)));
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->shifted.p, compat_rows.data(), compat_rows.size() * sizeof(int),
-                                      cudaMemcpyHostToDevice, st));
-    }
-    P->n_shifted = (int)compat_rows.size();
-    if (P->doublesided) {
-        const PlanSignal& S = P->sig[0];
-        FCWT_CUDA_TRY(P->Xs.ensure((size_t)S.sp.N * sizeof(float2)));
-        SigDesc s2 = sds[0];
-        s2.X = P->Xs.as<float2>();
-        if (S.log2R) FCWT_CUDA_TRY(P->Xsp.ensure((size_t)(S.sp.N / 2) * sizeof(float2)));
-        s2.Xp = S.log2R ? P->Xsp.as<float2>() : nullptr;
-        FCWT_CUDA_TRY(P->sigs2.ensure(sizeof(SigDesc)));
-        FCWT_CUDA_TRY(cudaMemcpyAsync(P->sigs2.p, &s2, sizeof(SigDesc), cudaMemcpyHostToDevice, st));
-        FCWT_CUDA_TRY(P->ds_tmp.ensure(std::max<size_t>((size_t)S.rows_out() * (size_t)S.n_out(), 1) * sizeof(float2)));
-    }
+    for (const auto& T : tabs)
+        FCWT_CUDA_TRY(launch_tc_tables(T.first[0], T.first[1], T.first[2], P->tc_tabs.as<unsigned char>() + T.second,
+                                       st));
+    FCWT_CUDA_TRY(launch_tc_weights(P->sigs.as<SigDesc>(), P->rows.as<RowDesc>(), owners.as<int>(),
+                                    (int)wts_rows.size(), P->pool.as<float>(), P->tc_wts.as<float>(), st));
     FCWT_CUDA_TRY(cudaStreamSynchronize(st));
     return FCWT_OK;
 }
@@ -738,9 +751,9 @@ void job_groups(const fcwt_plan* P, std::vector<std::pair<int, int>>& groups) {
 }
 
 // A pinned host buffer of at least `bytes` that no enqueued copy still reads.
-int upload_slot(fcwt_plan* P, size_t bytes, fcwt_plan::UploadSlot** out) {
-    fcwt_plan::UploadSlot& u = P->uploads[(size_t)P->upload_next];
-    P->upload_next = (P->upload_next + 1) % (int)P->uploads.size();
+int upload_slot(fcwt_context* ctx, size_t bytes, fcwt_context::UploadSlot** out) {
+    fcwt_context::UploadSlot& u = ctx->uploads[(size_t)ctx->upload_next];
+    ctx->upload_next = (ctx->upload_next + 1) % (int)ctx->uploads.size();
     if (u.pending) FCWT_CUDA_TRY(cudaEventSynchronize(u.done));
     u.pending = false;
     if (!u.done) FCWT_CUDA_TRY(cudaEventCreateWithFlags(&u.done, cudaEventDisableTiming));
@@ -869,8 +882,8 @@ int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* gr
         std::vector<std::pair<int, int>> groups;
         const FwdJob* djobs = graph_jobs;
         if (!djobs) {
-            fcwt_plan::UploadSlot* u = nullptr;
-            int rc = upload_slot(P, (size_t)nsig * sizeof(FwdJob), &u);
+            fcwt_context::UploadSlot* u = nullptr;
+            int rc = upload_slot(ctx, (size_t)nsig * sizeof(FwdJob), &u);
             if (rc) return rc;
             build_jobs(P, din, groups, static_cast<FwdJob*>(u->host));
             FCWT_CUDA_TRY(cudaMemcpyAsync(P->fwd_jobs.p, u->host, (size_t)nsig * sizeof(FwdJob),
@@ -1251,6 +1264,11 @@ int fcwt_context_destroy(fcwt_context* ctx) {
     ctx->counters.release();
     ctx->err.release();
     if (ctx->err_host) cudaFreeHost(ctx->err_host);
+    for (auto& u : ctx->uploads) {
+        if (u.pending && u.done) cudaEventSynchronize(u.done);
+        if (u.host) cudaFreeHost(u.host);
+        if (u.done) cudaEventDestroy(u.done);
+    }
     for (DevBuf* b : {&ctx->adj_tw, &ctx->adj_x, &ctx->adj_g, &ctx->adj_tmp, &ctx->adj_h, &ctx->adj_jobs,
                       &ctx->adj_rows, &ctx->adj_acc})
         b->release();
