@@ -81,6 +81,8 @@ SIGNATURES = {
     "fcwt_load_optimization_plan": (_i, [_vp, _i, _i, ctypes.c_char_p]),
     "fcwt_morlet_cwt_backward": (_i, [_vp, _vp, _i, _i, _f, _vp, _i, _f, _u, _vp, _vp,
                                       ctypes.POINTER(ctypes.c_double), _vp]),
+    "fcwt_morlet_power_backward": (_i, [_vp, _vp, _i, _i, _f, _vp, _i, _f, _u, _vp, _vp, _vp,
+                                      ctypes.POINTER(ctypes.c_double), _vp]),
     "fcwt_cwt_noalloc": (_i, [_vp, _i, _f, _vp, _i, _i, _u, _vp, _vp, ctypes.POINTER(_i)]),
 }
 

@@ -78,8 +78,9 @@ def _forward(ctx, x, sigma, freqs, fs: float, norm: bool, out_type: int):
     return y
 
 
-def _adjoint(ctx, x, G):
-    """(dL/dx, dL/dsigma, dL/dfreqs) for dL/dy = G (complex64 [batch, fn, n])."""
+def _adjoint(ctx, x, G, grad_p=None):
+    """(dL/dx, dL/dsigma, dL/dfreqs) for dL/dy = G (complex64 [batch, fn, n]),
+    or, with grad_p (float32, the same shape), dL/dy = 2 G grad_p."""
     B, n = x.shape
     F = ctx.f.size
     grad_x = torch.empty_like(x)
@@ -89,9 +90,10 @@ def _adjoint(ctx, x, G):
     c = _lib.context(x.device.index or 0)
     c.set_stream(torch.cuda.current_stream(x.device).cuda_stream)
     try:
-        _lib.call("fcwt_morlet_cwt_backward", c.handle, ctypes.c_void_p(x.data_ptr()), n, B,
+        _lib.call("fcwt_morlet_power_backward", c.handle, ctypes.c_void_p(x.data_ptr()), n, B,
                   ctypes.c_float(ctx.sig), ctypes.c_void_p(freqs32.ctypes.data), F, ctypes.c_float(ctx.fs),
                   _lib.FCWT_NORM if ctx.norm else 0, ctypes.c_void_p(G.data_ptr()),
+                  ctypes.c_void_p(grad_p.data_ptr() if grad_p is not None else None),
                   ctypes.c_void_p(grad_x.data_ptr()), ctypes.byref(gfb), ctypes.c_void_p(gf.ctypes.data))
     finally:
         c.set_stream(None)
@@ -127,10 +129,9 @@ class MorletPowerFunction(torch.autograd.Function):
         plan = _plan_for(x.device.index or 0, n, B, ctx.sig, ctx.scales, ctx.norm)
         y = torch.empty((B, ctx.f.size, n), dtype=torch.complex64, device=x.device)
         plan.execute([x[b] for b in range(B)], [y[b] for b in range(B)])
-        # dL/dy of L(|y|^2) in torch's convention for complex inputs: 2 y dL/dP
-        yr = torch.view_as_real(y)
-        yr.mul_((2.0 * grad_p.to(torch.float32)).unsqueeze(-1))
-        grad_x, gs, gfr = _adjoint(ctx, x, y)
+        # dL/dy of L(|y|^2) in torch's convention for complex inputs: 2 y dL/dP,
+        # formed by the adjoint kernels as they read y
+        grad_x, gs, gfr = _adjoint(ctx, x, y, grad_p.to(torch.float32).contiguous())
         return grad_x, gs, gfr, None, None
 
 

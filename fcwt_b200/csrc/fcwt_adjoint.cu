@@ -107,7 +107,7 @@ constexpr int kAdjColPitch = kP2 + 1;  // column pitch (float2) of the shared bu
 
 template <int M>
 __global__ void __launch_bounds__(kAdjFusedThreads, 1)
-    k_adjoint_rows(const float2* __restrict__ G, const float2* __restrict__ Xs, const AdjRow* __restrict__ rows,
+    k_adjoint_rows(const float2* __restrict__ G, const float* __restrict__ gain, const float2* __restrict__ Xs, const AdjRow* __restrict__ rows,
                    int n, int fn, const float2* __restrict__ tw, float cb, float amp, float inv_sigma,
                    float2* __restrict__ H, double* __restrict__ acc_sigma, double* __restrict__ acc_f) {
     constexpr int N = kP2 * M;
@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(kAdjFusedThreads, 1)
         const float2* __restrict__ g = G + ((size_t)b * fn + i) * (size_t)n;
         // (a) the row, conjugated, column-major: S[c][a] = conj(G[c + M a]), zero past n
         for (int t = tid; t < N; t += kAdjFusedThreads) {
-            const float2 v = t < n ? __ldcs(g + t) : make_float2(0.0f, 0.0f);
+            float2 v = t < n ? __ldcs(g + t) : make_float2(0.0f, 0.0f);
+            // power layer: dL/dy = 2 y dL/dP on the fly (one pass over y and dL/dP instead
+            // of three over y in a separate kernel)
+            if (gain && t < n) v = cscale(v, 2.0f * __ldcs(gain + ((size_t)b * fn + i) * (size_t)n + t));
             S[(t & (M - 1)) * kAdjColPitch + (t >> LOGM)] = make_float2(v.x, -v.y);
         }
         __syncthreads();
@@ -264,7 +267,7 @@ size_t adjoint_fused_smem(int M) { return sizeof(float2) * ((size_t)M * dev::kAd
 
 // The fused row adjoint for N = 1024 M, M in {1, 2, 4, 8, 16}; returns
 // cudaErrorInvalidValue for other N (the caller then uses the FFT passes).
-cudaError_t launch_adjoint_rows(const float2* G, const float2* Xs, const void* rows, int n, int log2N, int fn,
+cudaError_t launch_adjoint_rows(const float2* G, const float* gain, const float2* Xs, const void* rows, int n, int log2N, int fn,
                                 int batch, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
                                 double* acc_sigma, double* acc_f, cudaStream_t st) {
     const int M = log2N >= kLog2P2 ? 1 << (log2N - kLog2P2) : 0;
@@ -277,7 +280,7 @@ cudaError_t launch_adjoint_rows(const float2* G, const float2* Xs, const void* r
     case MM:                                                                                                \
         e = cudaFuncSetAttribute(dev::k_adjoint_rows<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
         if (e != cudaSuccess) return e;                                                                     \
-        dev::k_adjoint_rows<MM><<<grid, dev::kAdjFusedThreads, sm, st>>>(G, Xs, r, n, fn, tw, cb, amp, inv_sigma, \
+        dev::k_adjoint_rows<MM><<<grid, dev::kAdjFusedThreads, sm, st>>>(G, gain, Xs, r, n, fn, tw, cb, amp, inv_sigma, \
                                                                           H, acc_sigma, acc_f);             \
         break;
     switch (M) {

@@ -39,7 +39,10 @@ cudaError_t launch_adjoint_accum(const float2* Xs, const float2* Gh, float2* H, 
 cudaError_t launch_take_real(const float2* Y, long long Nstride, int n, int batch, float scale, float* gx,
                              cudaStream_t st);
 int adjoint_rows_per_pass();
-cudaError_t launch_adjoint_rows(const float2* G, const float2* Xs, const void* rows, int n, int log2N, int fn,
+cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int rows, const float2* Xs, const void* rowc,
+                                int log2N, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
+                                double* acc_sigma, double* acc_f, cudaStream_t st);
+cudaError_t launch_adjoint_rows(const float2* G, const float* gain, const float2* Xs, const void* rows, int n, int log2N, int fn,
                                 int batch, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
                                 double* acc_sigma, double* acc_f, cudaStream_t st);
 cudaError_t engine_configure();
@@ -789,6 +792,7 @@ void build_jobs(fcwt_plan* P, const void* const* din, std::vector<std::pair<int,
             j.n = S.sp.n;
             j.log2R = S.log2R;
             j.Xp = S.Xp.as<float2>();
+            j.gain = nullptr;
             j.X = S.X.as<float2>();
             j.tmp = P->fwd_tmp.as<float2>() + tmp_off[(size_t)s];
         }
@@ -1744,6 +1748,13 @@ int fcwt_ccwt(fcwt_context* ctx, const float* input, int n, float fb, const floa
 int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch, float fb, const float* freqs,
                              int fn, float fs, unsigned flags, const void* grad_out, float* grad_x, double* grad_fb,
                              double* grad_freqs) {
+    return fcwt_morlet_power_backward(ctx, x, n, batch, fb, freqs, fn, fs, flags, grad_out, nullptr, grad_x, grad_fb,
+                                      grad_freqs);
+}
+
+int fcwt_morlet_power_backward(fcwt_context* ctx, const float* x, int n, int batch, float fb, const float* freqs,
+                               int fn, float fs, unsigned flags, const void* grad_out, const float* grad_power,
+                               float* grad_x, double* grad_fb, double* grad_freqs) {
     using namespace fcwt;
     int rc = ctx_prepare(ctx);
     if (rc) return rc;
@@ -1755,8 +1766,10 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
     if (n == 0 || batch == 0) return FCWT_OK;
     if (!x || !grad_out || !grad_x || (fn > 0 && !freqs))
         return fail(FCWT_ERR_INVALID, "null pointer argument");
-    rc = check_pointer_devices({x, grad_out, grad_x}, ctx->device);
+    rc = check_pointer_devices({x, grad_out, grad_x, grad_power}, ctx->device);
     if (rc) return rc;
+    if (grad_power && !is_device_pointer(grad_power))
+        return fail(FCWT_ERR_INVALID, "grad_power must be a device pointer");
     if (!is_device_pointer(x) || !is_device_pointer(grad_out) || !is_device_pointer(grad_x))
         return fail(FCWT_ERR_INVALID, "x, grad_out and grad_x must be device pointers");
     const int log2N = host::find2power(n);
@@ -1769,7 +1782,14 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
         return FCWT_OK;
     }
     const int half = N / 2;
-    const int RP = adjoint_rows_per_pass();
+    // N = 1024 .. 16384: one kernel, rows in shared memory; longer: two passes, the
+    // second fused with the sums, over as many rows as keep the first pass's results
+    // in L2 (64 MB); shorter: whole spectra, a few rows at a time
+    const bool fused = log2N >= kLog2P2 && log2N <= kLog2P2 + 4;
+    const bool long_rows = log2N > kLog2P2 + 4;
+    const int RP = long_rows ? (int)std::max<size_t>(1, std::min<size_t>((size_t)fn, ((size_t)64 << 20) /
+                                                                                  ((size_t)batch * N * sizeof(float2))))
+                             : adjoint_rows_per_pass();
     const int nchunks = (fn + RP - 1) / RP;
     // tables
     if (ctx->adj_tw_log2N != log2N) {
@@ -1780,8 +1800,8 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
     const size_t BN = (size_t)batch * N;
     FCWT_CUDA_TRY(ctx->adj_x.ensure(BN * sizeof(float2)));
     FCWT_CUDA_TRY(ctx->adj_h.ensure(BN * sizeof(float2)));
-    FCWT_CUDA_TRY(ctx->adj_g.ensure(BN * RP * sizeof(float2)));
-    FCWT_CUDA_TRY(ctx->adj_tmp.ensure(BN * RP * sizeof(float2)));
+    FCWT_CUDA_TRY(ctx->adj_g.ensure(BN * (fused || long_rows ? 1 : RP) * sizeof(float2)));
+    FCWT_CUDA_TRY(ctx->adj_tmp.ensure(BN * (fused ? 1 : RP) * sizeof(float2)));
     const size_t njobs_total = (size_t)batch * (2 + (size_t)fn);
     FCWT_CUDA_TRY(ctx->adj_jobs.ensure(njobs_total * sizeof(FwdJob)));
     if (ctx->adj_jobs_host_bytes < njobs_total * sizeof(FwdJob)) {
@@ -1825,6 +1845,7 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
         j.n = n;
         j.log2R = 0;
         j.Xp = nullptr;
+        j.gain = nullptr;
         j.X = ctx->adj_x.as<float2>() + (size_t)b * N;
         j.tmp = ctx->adj_tmp.as<float2>() + (size_t)b * N;
     }
@@ -1834,9 +1855,9 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
     jo += batch;
     // rows in chunks: Ghat = FFT(G), accumulate H and the parameter sums
     const float2* G = static_cast<const float2*>(grad_out);
-    const bool fused = log2N >= kLog2P2 && log2N <= kLog2P2 + 4;  // N = 1024 .. 16384: one kernel, in SMEM
+    auto grow = [&](int b, int i) { return grad_power ? grad_power + ((size_t)b * fn + i) * n : nullptr; };
     if (fused) {
-        FCWT_CUDA_TRY(launch_adjoint_rows(G, ctx->adj_x.as<float2>(), ctx->adj_rows.p, n, log2N, fn, batch, tw,
+        FCWT_CUDA_TRY(launch_adjoint_rows(G, grad_power, ctx->adj_x.as<float2>(), ctx->adj_rows.p, n, log2N, fn, batch, tw,
                                           (float)(two_pi * fb), host::mother_norm(), 1.0f / fb,
                                           ctx->adj_h.as<float2>(), ctx->adj_acc.as<double>(),
                                           ctx->adj_acc.as<double>() + 1, st));
@@ -1852,12 +1873,23 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
                 j.in_c = G + ((size_t)b * fn + i0 + i) * n;
                 j.n = n;
                 j.log2R = 0;
-        j.Xp = nullptr;
+                j.Xp = nullptr;
+                j.gain = grow(b, i0 + i);
                 j.X = ctx->adj_g.as<float2>() + ((size_t)b * nr + i) * N;
                 j.tmp = ctx->adj_tmp.as<float2>() + ((size_t)b * nr + i) * N;
             }
         }
         FCWT_CUDA_TRY(cudaMemcpyAsync(jd + jo, jh + jo, (size_t)batch * nr * sizeof(FwdJob), cudaMemcpyHostToDevice, st));
+        if (long_rows) {
+            FCWT_CUDA_TRY(launch_adjoint_long(jd + jo, ctx->adj_tmp.as<float2>(), batch, nr, ctx->adj_x.as<float2>(),
+                                              static_cast<const AdjRowH*>(ctx->adj_rows.p) + i0, log2N, tw,
+                                              (float)(two_pi * fb), host::mother_norm(), 1.0f / fb,
+                                              ctx->adj_h.as<float2>(), ctx->adj_acc.as<double>(),
+                                              ctx->adj_acc.as<double>() + 1 + i0, st));
+            ctx->kernel_launches += 2;
+            jo += (size_t)batch * nr;
+            continue;
+        }
         FCWT_CUDA_TRY(launch_forward_batched(jd + jo, batch * nr, log2N, tw, st, &nk, false));
         ctx->kernel_launches += nk;
         jo += (size_t)batch * nr;
@@ -1875,6 +1907,7 @@ int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch
         j.n = N;
         j.log2R = 0;
         j.Xp = nullptr;
+        j.gain = nullptr;
         j.X = ctx->adj_g.as<float2>() + (size_t)b * N;
         j.tmp = ctx->adj_tmp.as<float2>() + (size_t)b * N;
     }

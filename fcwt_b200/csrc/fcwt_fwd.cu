@@ -40,13 +40,15 @@ constexpr int kFftTargetCtas = 2 * 148;  // about two CTAs per SM of a B200
 // Element idx of a signal with implicit zero padding: a complex sample, or
 // (r2c) the real pair (x[2 idx], x[2 idx + 1]).
 __device__ __forceinline__ float2 fwd_input(const float* __restrict__ in_r, const float2* __restrict__ in_c,
-                                            int n_in, int idx, int r2c) {
+                                            const float* __restrict__ gain, int n_in, int idx, int r2c) {
     if (in_r && r2c) {
         const int i0 = 2 * idx;
         return make_float2(i0 < n_in ? __ldg(in_r + i0) : 0.0f, i0 + 1 < n_in ? __ldg(in_r + i0 + 1) : 0.0f);
     }
     if (idx >= n_in) return make_float2(0.0f, 0.0f);
-    return in_r ? make_float2(__ldg(in_r + idx), 0.0f) : __ldg(in_c + idx);
+    if (in_r) return make_float2(__ldg(in_r + idx), 0.0f);
+    const float2 v = __ldg(in_c + idx);
+    return gain ? cscale(v, 2.0f * __ldg(gain + idx)) : v;
 }
 
 // w_T^{SIGN e} from the two-level table of T = 2^log2T (which holds w_T^{+e}).
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
         }
         const int col = c0 + cc;
         const int j = mode == 0 ? col + (i << log2S) : (col << log2L) + i;
-        a[(i << log2B) + cc] = src_sel == 0 ? fwd_input(J.in_r, J.in_c, J.n, j, r2c) : src[j];
+        a[(i << log2B) + cc] = src_sel == 0 ? fwd_input(J.in_r, J.in_c, J.gain, J.n, j, r2c) : src[j];
     }
     __syncthreads();
     const float2* res = smem_fft<SIGN>(a, b, log2L, log2B, tl, th);
@@ -171,6 +173,102 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
         const int o = col + (k << log2S);
         dst[o] = v;
         if (dst_sel == 1 && J.log2R && o < (1 << (log2C - 1))) J.Xp[perm_bin(o, J.log2R)] = v;
+    }
+}
+
+// ---- adjoint of the differentiable transform, N > 16384: pass B of the incoming
+// gradient rows' FFTs and their use in one kernel. A CTA takes B columns k2 of
+// the rows [r0, r0 + rows) of signal blockIdx.y: it transforms each row's columns
+// in shared memory and adds, for its bins q = k2 + C2 k1 < N / 2, g_i(q) Ghat to H
+// (in registers over its rows) and the sigma and frequency partial sums, so the
+// rows' spectra are never written. (Writing them and reading them back took the
+// second pass 43 us and the sums 11 us per 64 rows of N = 65536.)
+constexpr int kAdjColPos = (1 << kFftMaxLog2Tile) / 2 / kFftThreads;  // bins per thread, at most
+
+__global__ void __launch_bounds__(kFftThreads)
+    k_adjoint_cols(const float2* __restrict__ T, const float2* __restrict__ Xs, const float2* __restrict__ rowc,
+                   int rows_total, int rows_per_cta, int log2C, int log2L, int log2B, const float2* __restrict__ tw,
+                   float cb, float amp, float inv_sigma, float2* __restrict__ H, double* __restrict__ acc_sigma,
+                   double* __restrict__ acc_f) {
+    extern __shared__ float2 fft_sm[];
+    __shared__ float2 tl[64], th[64];
+    __shared__ float s_red[kFftThreads / 32][2];
+    const int L = 1 << log2L, B = 1 << log2B;
+    const int log2S = log2C - log2L;
+    const int tot = L << log2B;
+    const int pos = tot >> 1;  // bins below N / 2
+    const int c0 = blockIdx.x << log2B;
+    const int b = blockIdx.y;
+    const int r0 = blockIdx.z * rows_per_cta;
+    const int nr = min(rows_per_cta, rows_total - r0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = threadIdx.x; t < 128; t += kFftThreads) {
+        const unsigned e = t < 64 ? (unsigned)t : (unsigned)(t - 64) << 6;
+        if (e < (unsigned)L) (t < 64 ? tl[t] : th[t - 64]) = fft_tw<-1>(tw, log2C, e << (log2C - log2L));
+    }
+    float2 h[kAdjColPos], xq[kAdjColPos];
+#pragma unroll
+    for (int i = 0; i < kAdjColPos; i++) {
+        const int t = threadIdx.x + i * kFftThreads;
+        h[i] = make_float2(0.0f, 0.0f);
+        if (t < pos) {
+            const int q = c0 + (t & (B - 1)) + ((t >> log2B) << log2S);
+            xq[i] = __ldg(Xs + ((size_t)b << log2C) + q);
+        }
+    }
+    double dsig = 0.0;
+    for (int r = 0; r < nr; r++) {
+        const float2* __restrict__ src = T + (((size_t)b * rows_total + r0 + r) << log2C) + ((size_t)c0 << log2L);
+        float2* a = fft_sm;
+        __syncthreads();
+        for (int t = threadIdx.x; t < tot; t += kFftThreads) a[((t & (L - 1)) << log2B) + (t >> log2L)] = __ldcg(src + t);
+        __syncthreads();
+        const float2* res = smem_fft<-1>(a, fft_sm + tot, log2L, log2B, tl, th);
+        const float2 rc = __ldg(rowc + r0 + r);  // (ca, dfdq)
+        float ds = 0.0f, df = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kAdjColPos; i++) {
+            const int t = threadIdx.x + i * kFftThreads;
+            if (t < pos) {
+                const float qf = (float)(c0 + (t & (B - 1)) + ((t >> log2B) << log2S));
+                const float u = rc.x * qf - cb;
+                const float g = amp * expf(-0.5f * u * u);
+                const float2 gh = res[t];
+                h[i].x += g * gh.x;
+                h[i].y += g * gh.y;
+                const float re = xq[i].x * gh.x + xq[i].y * gh.y;  // Re(X conj(Gh))
+                ds += -g * u * u * inv_sigma * re;
+                df += g * u * rc.y * qf * re;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            ds += __shfl_xor_sync(0xffffffffu, ds, o);
+            df += __shfl_xor_sync(0xffffffffu, df, o);
+        }
+        if (lane == 0) {
+            s_red[warp][0] = ds;
+            s_red[warp][1] = df;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double d = 0.0;
+            for (int w = 0; w < kFftThreads / 32; w++) {
+                dsig += (double)s_red[w][0];
+                d += (double)s_red[w][1];
+            }
+            atomicAdd(acc_f + r0 + r, d);
+        }
+    }
+    if (threadIdx.x == 0) atomicAdd(acc_sigma, dsig);
+#pragma unroll
+    for (int i = 0; i < kAdjColPos; i++) {
+        const int t = threadIdx.x + i * kFftThreads;
+        if (t < pos) {
+            float* hp = reinterpret_cast<float*>(H + ((size_t)b << log2C) + c0 + (t & (B - 1)) + ((t >> log2B) << log2S));
+            atomicAdd(hp, h[i].x);
+            atomicAdd(hp + 1, h[i].y);
+        }
     }
 }
 
@@ -213,6 +311,8 @@ __global__ void k_r2c_split(const FwdJob* __restrict__ jobs, FwdJob one, int log
 cudaError_t fft_configure() {
     cudaError_t e = cudaFuncSetAttribute(dev::k_fft_cols<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          dev::kFftSmemBytes);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(dev::k_adjoint_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kFftSmemBytes);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(dev::k_fft_cols<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kFftSmemBytes);
 }
@@ -287,6 +387,7 @@ cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log
     one.X = out;
     one.tmp = tmp;
     one.Xp = Xp;
+    one.gain = nullptr;
     return fft_signals<-1>(nullptr, one, 1, log2N, tw, in_r != nullptr, st, n_kernels);
 }
 
@@ -294,6 +395,30 @@ cudaError_t launch_forward_batched(const FwdJob* jobs, int njobs, int log2N, con
                                    int* n_kernels, bool real) {
     FwdJob none{};
     return fft_signals<-1>(jobs, none, njobs, log2N, tw, real, st, n_kernels);
+}
+
+// The adjoint's row FFTs for N > 16384: pass A of `njobs` = batch x rows gradient
+// rows into consecutive tmp buffers (N values each, from `tmp`), then the fused
+// pass B. rowc: (ca, dfdq) of the rows.
+cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int rows, const float2* Xs, const void* rowc,
+                                int log2N, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
+                                double* acc_sigma, double* acc_f, cudaStream_t st) {
+    const int log2C2 = log2N / 2, log2C1 = log2N - log2C2;
+    FwdJob none{};
+    int log2B = std::min(3, dev::kFftMaxLog2Tile - log2C2);
+    dev::k_fft_cols<-1><<<dim3(1u << (log2C1 - log2B), (unsigned)(batch * rows)), dev::kFftThreads,
+                          (size_t)16 << (log2C2 + log2B), st>>>(jobs, none, 0, 2, log2N, log2C2, log2B, 0, 0, tw, log2N);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    log2B = std::min(3, dev::kFftMaxLog2Tile - log2C1);
+    const int groups = 1 << (log2C2 - log2B);
+    // rows per CTA: enough CTAs for every SM, H added once per CTA
+    int per = 1;
+    while (per < 16 && per < rows && (long long)groups * batch * ((rows + 2 * per - 1) / (2 * per)) >= 8 * 148) per *= 2;
+    dev::k_adjoint_cols<<<dim3(groups, batch, (rows + per - 1) / per), dev::kFftThreads, (size_t)16 << (log2C1 + log2B),
+                          st>>>(tmp, Xs, static_cast<const float2*>(rowc), rows, per, log2N, log2C1, log2B, tw, cb, amp,
+                                inv_sigma, H, acc_sigma, acc_f);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_inverse_batched(const FwdJob* jobs, int njobs, int log2N, const float2* tw, cudaStream_t st,

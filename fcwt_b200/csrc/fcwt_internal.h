@@ -101,6 +101,7 @@ struct FwdJob {
     float2* X;
     float2* tmp;
     float2* Xp;
+    const float* gain;  // complex inputs: sample i is 2 gain[i] in_c[i] (null: in_c[i])
 };
 
 // Position of bin q in the permuted spectrum copy: within its block of P2 = 16 R

@@ -219,6 +219,13 @@ int fcwt_plan_execute_graph(fcwt_plan* plan, const void* const* inputs, void* co
 int fcwt_morlet_cwt_backward(fcwt_context* ctx, const float* x, int n, int batch, float fb, const float* freqs,
                              int fn, float fs, unsigned flags, const void* grad_out, float* grad_x, double* grad_fb,
                              double* grad_freqs);
+/* The same for an upstream gradient of P = |y|^2: grad_out holds y itself (the
+ * complex64 transform, [batch][fn][n]) and grad_power dL/dP (float32, the same
+ * shape, device memory); dL/dy = 2 y dL/dP is formed as y is read. grad_power
+ * null: grad_out is dL/dy. */
+int fcwt_morlet_power_backward(fcwt_context* ctx, const float* x, int n, int batch, float fb, const float* freqs,
+                               int fn, float fs, unsigned flags, const void* grad_out, const float* grad_power,
+                               float* grad_x, double* grad_fb, double* grad_freqs);
 
 /* ---- tuning files
  * FCWT::create_FFT_optimization_plan(maxsize, flags), src/fcwt/fcwt.cpp:313-374:

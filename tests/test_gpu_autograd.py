@@ -174,3 +174,39 @@ def test_power_layer_module():
     assert torch.allclose(P.detach(), y.detach().abs() ** 2, rtol=1e-5, atol=1e-7 * float(P.detach().max()))
     (-P.mean()).backward()
     assert float(lp.freqs.grad[0]) < 0 < float(lp.freqs.grad[1])
+
+
+# the long-signal adjoint: smallest N (32768, C1 = 256, C2 = 128), a square split
+# (65536), several passes of rows (the 64 MB limit), one row, more rows than a CTA takes
+@pytest.mark.parametrize("n,B,F", [(16385, 1, 1), (32768, 3, 5), (50000, 2, 40), (65537, 5, 19), (300000, 1, 33)])
+@pytest.mark.parametrize("power", [False, True])
+def test_long_adjoint_edges(n, B, F, power):
+    """Gradients of a fixed linear functional against float64 autograd. Relative
+    bound 2e-5: the FP32 operator's own 1e-6 plus sums of n F float products
+    whose partial sums are float only over one thread's bins and a warp."""
+    import torch
+
+    from fcwt_b200.autograd import morlet_cwt, morlet_power_cwt
+
+    g = torch.Generator(device="cuda").manual_seed(n + F)
+    fs = 1000.0
+    t = torch.arange(n, dtype=torch.float64, device="cuda") / fs
+    x0 = torch.sin(2 * math.pi * 40.0 * t)[None] + 0.3 * torch.randn((B, n), generator=g, device="cuda", dtype=torch.float64)
+    f0 = torch.from_numpy(np.geomspace(8.0, 120.0, F)).cuda()
+    x = x0.float().requires_grad_(True)
+    sigma = torch.tensor(2.0, device="cuda", requires_grad=True)
+    freqs = f0.float().requires_grad_(True)
+    xr = x.detach().double().requires_grad_(True)
+    sr = torch.tensor(2.0, dtype=torch.float64, device="cuda", requires_grad=True)
+    fr = freqs.detach().double().requires_grad_(True)
+    yr = ref_forward(xr, sr, fr, fs, True)
+    if power:
+        G = 1.0 + torch.rand((B, F, n), generator=g, device="cuda")
+        got = torch.autograd.grad(morlet_power_cwt(x, sigma, freqs, fs), [x, sigma, freqs], G)
+        want = torch.autograd.grad(yr.real.square() + yr.imag.square(), [xr, sr, fr], G.double())
+    else:
+        G = yr.detach().to(torch.complex64)
+        got = torch.autograd.grad(morlet_cwt(x, sigma, freqs, fs), [x, sigma, freqs], G)
+        want = torch.autograd.grad(yr, [xr, sr, fr], G.to(torch.complex128))
+    for a, b in zip(got, want):
+        assert float(torch.linalg.vector_norm(a.double() - b)) <= 2e-5 * float(torch.linalg.vector_norm(b))
