@@ -83,10 +83,21 @@ __device__ __forceinline__ void smem_stage(const float2* __restrict__ in, float2
         const int k = j & ((1 << log2Ns) - 1);
         float2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            float2 x = in[((j + r * Lr) << log2B) + cc];
-            if (r > 0 && k > 0) x = cmul(x, stage_tw(tl, th, (unsigned)(r * k) << shift));
-            v[r] = x;
+        for (int r = 0; r < R; r++) v[r] = in[((j + r * Lr) << log2B) + cc];
+        if (k > 0) {
+            // w^r: powers of two from the tables, the others as products of at most
+            // four of them (15 lookups of a radix-16 task kept the load unit busy)
+            float2 w[R];
+#pragma unroll
+            for (int r = 1; r < R; r++) {
+                constexpr int top = R;
+                int hb = 1;
+#pragma unroll
+                for (int q = 1; q < top; q *= 2)
+                    if (q <= r) hb = q;
+                w[r] = hb == r ? stage_tw(tl, th, (unsigned)(r * k) << shift) : cmul(w[hb], w[r - hb]);
+                v[r] = cmul(v[r], w[r]);
+            }
         }
         fft_reg<R, SIGN>(v);
         const int base = (j - k) * R + k;
@@ -163,13 +174,24 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
     __syncthreads();
     const float2* res = smem_fft<SIGN>(a, b, log2L, log2B, tl, th);
     float2* dst = dst_sel == 1 ? J.X : J.tmp;
-    for (int t = threadIdx.x; t < tot; t += kFftThreads) {
+    // inter-pass twiddle w_C^{SIGN col k}: a thread's column is fixed and its k goes up
+    // by 128 / B, so the twiddle advances by a factor; looked up again every four
+    // (scattered lookups of both tables at each sample took most of the pass: 94 us
+    // for 128 rows of 65536)
+    const int dk = kFftThreads >> log2B;
+    const int my_col = c0 + (threadIdx.x & (B - 1));
+    float2 w = make_float2(1.0f, 0.0f), wstep = w;
+    if (mode == 0) wstep = fft_tw<SIGN>(tw, log2T, (unsigned)(my_col * dk) << (log2T - log2C));
+    int it = 0;
+    for (int t = threadIdx.x; t < tot; t += kFftThreads, it++) {
         const int cc = t & (B - 1);
         const int k = t >> log2B;
         const int col = c0 + cc;
         float2 v = res[t];
-        if (mode == 0 && col > 0 && k > 0)
-            v = cmul(v, fft_tw<SIGN>(tw, log2T, (unsigned)(col * k) << (log2T - log2C)));
+        if (mode == 0) {
+            w = (it & 3) ? cmul(w, wstep) : fft_tw<SIGN>(tw, log2T, (unsigned)(col * k) << (log2T - log2C));
+            v = cmul(v, w);
+        }
         const int o = col + (k << log2S);
         dst[o] = v;
         if (dst_sel == 1 && J.log2R && o < (1 << (log2C - 1))) J.Xp[perm_bin(o, J.log2R)] = v;
