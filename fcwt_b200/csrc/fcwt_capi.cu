@@ -50,6 +50,9 @@ cudaError_t engine_blocks_per_sm(int* out);
 cudaError_t launch_engine(const EngineParams& p, int grid, cudaStream_t st);
 cudaError_t launch_engine(const EngineParams& p, const CUtensorMap& omap, int grid, cudaStream_t st);
 cudaError_t tc_configure();
+cudaError_t small_configure();
+cudaError_t launch_rows_small(const SigDesc* sigs, const RowDesc* rows, const int* list, int n_list, const float* pool,
+                              const OutPtrs& outs, int out_type, int log2L, cudaStream_t st);
 cudaError_t launch_tc_weights(const SigDesc* sigs, const RowDesc* rows, const int* row_list, int n_list,
                               const float* pool, float* wts, cudaStream_t st);
 size_t tc_table_bytes();
@@ -290,11 +293,12 @@ struct fcwt_plan {
     bool is_complex = false;
     std::vector<PlanSignal> sig;
     std::vector<PlanTables> tables;
-    DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, tc_wts, tc_tabs;
+    DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, small_rows, tc_wts, tc_tabs;
     DevBuf tc_units;  // work list of the tensor-core engine (rows, the last ones possibly split)
     int n_units[2] = {0, 0};  // units of R = 16 and, after them, of R = 8
     DevBuf mem;  // one allocation that holds the buffers plan_build fills
     int n_items = 0;
+    int n_small = 0, small_log2L = 0;  // rows of N <= kMaxFusedN, log2 of their largest N / dec
     int n_rows = 0;
     int n_tc = 0;  // rows run by the tensor-core engine
     std::vector<float> custom_mother;  // caller's wavelet table (N floats), empty for Morlet(fb)
@@ -342,6 +346,7 @@ void plan_release(fcwt_plan* p) {
     p->fwd_tmp.release();
     p->graph_jobs.release();
     p->tc_rows.release();
+    p->small_rows.release();
     p->tc_units.release();
     p->tc_wts.release();
     p->tc_tabs.release();
@@ -467,6 +472,8 @@ int plan_build(fcwt_plan* P) {
     std::vector<RowDesc> rows;
     std::vector<int> two_phase_rows;  // global indices, in order
     std::vector<int> tc_rows;         // rows of the tensor-core engine, in order
+    std::vector<int> small_rows;      // rows of N <= kMaxFusedN
+    int max_small_log2L = 0;          // log2 of their largest transform length N / dec
     long long tc_wts_elems = 0;       // size of their weight table
     std::vector<int> wts_rows;        // rows that own a weight-table entry
     std::map<std::array<uint32_t, 12>, long long> wts_owner;
@@ -592,7 +599,8 @@ int plan_build(fcwt_plan* P) {
                 two_phase_rows.push_back(g);
                 max_two_phase_log2N = std::max(max_two_phase_log2N, sp.log2N);
             } else {
-                items.push_back({sp.N < kP2 ? ITEM_SMALL : ITEM_FUSED, g, 0, 0});
+                small_rows.push_back(g);
+                max_small_log2L = std::max(max_small_log2L, std::max(0, sp.log2N - (31 - __builtin_clz((unsigned)d.dec))));
             }
         }
     }
@@ -634,6 +642,8 @@ int plan_build(fcwt_plan* P) {
     }
     P->n_items = (int)items.size();
     P->n_tc = (int)tc_rows.size();
+    P->n_small = (int)small_rows.size();
+    P->small_log2L = max_small_log2L;
 
     P->n_shifted = (int)compat_rows.size();
     std::vector<int> units;
@@ -662,6 +672,7 @@ int plan_build(fcwt_plan* P) {
     want.push_back({&P->rows, rows.size() * sizeof(RowDesc)});
     want.push_back({&P->items, items.size() * sizeof(Item)});
     want.push_back({&P->tc_rows, tc_rows.size() * sizeof(int)});
+    want.push_back({&P->small_rows, small_rows.size() * sizeof(int)});
     want.push_back({&P->tc_units, units.size() * sizeof(int)});
     want.push_back({&owners, wts_rows.size() * sizeof(int)});
     want.push_back({&P->shifted, compat_rows.size() * sizeof(int)});
@@ -671,7 +682,7 @@ int plan_build(fcwt_plan* P) {
     for (auto& T : P->tables) {
         const size_t N = (size_t)1 << T.log2N;
         want.push_back({&T.mother, N * sizeof(float)});
-        want.push_back({&T.tw, (1024 + std::max<size_t>(N / kP2, 1)) * sizeof(float2)});
+        want.push_back({&T.tw, (size_t)tw_entries((int)N) * sizeof(float2)});
     }
     for (auto& S : P->sig) {
         want.push_back({&S.X, (size_t)S.sp.N * sizeof(float2)});
@@ -714,8 +725,8 @@ int plan_build(fcwt_plan* P) {
     sd2 = sds[0];
     sd2.X = P->Xs.as<float2>();
     sd2.Xp = P->sig[0].log2R ? P->Xsp.as<float2>() : nullptr;
-    const void* src[] = {pool.data(),  sds.data(),      rows.data(),        items.data(), tc_rows.data(),
-                         units.data(), wts_rows.data(), compat_rows.data(), &sd2};
+    const void* src[] = {pool.data(),       sds.data(),   rows.data(),     items.data(),       tc_rows.data(),
+                         small_rows.data(), units.data(), wts_rows.data(), compat_rows.data(), &sd2};
     std::vector<char> image(filled);
     for (size_t i = 0; i < n_filled; i++)
         if (want[i].second)
@@ -967,6 +978,13 @@ int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, in
             ctx->kernel_launches += 1;
         }
     }
+    if (P->n_small > 0) {
+        OutPtrs outs;
+        std::memcpy(outs.p, ep.outs, sizeof(outs.p));
+        FCWT_CUDA_TRY(launch_rows_small(ep.sigs, ep.rows, P->small_rows.as<int>(), P->n_small, ep.stale_pool, outs,
+                                        out_type, P->small_log2L, st));
+        ctx->kernel_launches += 1;
+    }
     if (P->n_items > 0) {
         FCWT_CUDA_TRY(launch_engine(ep, omap, grid, st));
         ctx->kernel_launches += 1;
@@ -983,7 +1001,7 @@ int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, in
 constexpr size_t kPipeBlockBytes = 256ull << 20;
 
 bool pipeline_applies(const fcwt_plan* P, size_t out_bytes) {
-    return P->sig.size() == 1 && P->n_items == 0 && P->n_tc == P->n_rows && !P->doublesided &&
+    return P->sig.size() == 1 && P->n_tc == P->n_rows && !P->doublesided &&
            P->n_shifted == 0 && out_bytes > kPipeBlockBytes;
 }
 
@@ -1233,6 +1251,7 @@ int fcwt_context_create(int device, fcwt_context** out) {
     if (e == cudaSuccess) e = cudaMallocHost(&c->err_host, sizeof(int));
     if (e == cudaSuccess) e = fcwt::engine_configure();
     if (e == cudaSuccess) e = fcwt::tc_configure();
+    if (e == cudaSuccess) e = fcwt::small_configure();
     int per_sm = 0;
     if (e == cudaSuccess) e = fcwt::engine_blocks_per_sm(&per_sm);
     c->engine_ctas = std::max(1, per_sm) * c->num_sms;
@@ -1793,7 +1812,7 @@ int fcwt_morlet_power_backward(fcwt_context* ctx, const float* x, int n, int bat
     const int nchunks = (fn + RP - 1) / RP;
     // tables
     if (ctx->adj_tw_log2N != log2N) {
-        FCWT_CUDA_TRY(ctx->adj_tw.ensure((size_t)(1024 + std::max(N / 1024, 1)) * sizeof(float2)));
+        FCWT_CUDA_TRY(ctx->adj_tw.ensure((size_t)tw_entries(N) * sizeof(float2)));
         FCWT_CUDA_TRY(launch_twiddle(log2N, ctx->adj_tw.as<float2>(), st));
         ctx->adj_tw_log2N = log2N;
     }

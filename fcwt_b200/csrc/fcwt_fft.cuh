@@ -138,10 +138,12 @@ __device__ __forceinline__ void dft1024_warp_xor(float2 (&x)[32], int lane, floa
 }
 
 // w_N^e from the two-level table of a transform length N = 2^log2N:
-// tw[0..1023] = w_N^j, tw[1024 + j] = w_N^{1024 j}. SIGN < 0 conjugates.
+// tw[0..1023] = w_N^j, tw[1024 + j] = w_N^{1024 j}; for 1024 < N <= 8192 all N
+// factors follow (tw_entries).
 __device__ __forceinline__ float2 tw_lookup(const float2* __restrict__ tw, int log2N, unsigned e) {
-    if (log2N <= 10) return __ldg(tw + (e & ((1u << log2N) - 1)));
     e &= (1u << log2N) - 1;
+    if (log2N <= 10) return __ldg(tw + e);
+    if (log2N <= 13) return __ldg(tw + 1024 + (1 << (log2N - 10)) + e);
     return cmul(__ldg(tw + (e & 1023u)), __ldg(tw + 1024 + (e >> 10)));
 }
 

@@ -59,10 +59,18 @@ __device__ __forceinline__ float2 fft_tw(const float2* __restrict__ tw, int log2
     return w;
 }
 
-// w_L^{SIGN e}, e < L, from the CTA's two-level table of w_L^{SIGN j}:
-// tl[j] for j < 64 and th[j] = w_L^{SIGN 64 j} for j < L / 64.
-__device__ __forceinline__ float2 stage_tw(const float2* __restrict__ tl, const float2* __restrict__ th, unsigned e) {
-    return e < 64u ? tl[e] : cmul(tl[e & 63u], th[e >> 6]);
+// Stage twiddles of a CTA: w_L^{SIGN j} for j < min(L, 1024); for longer L the factors
+// w_L^{SIGN 1024 j} follow.
+constexpr int kStageTw = 1024 + (1 << kFftMaxLog2Tile) / 1024;
+template <int SIGN>
+__device__ __forceinline__ void stage_tw_fill(float2* __restrict__ tl, const float2* __restrict__ tw, int log2T,
+                                              int log2L) {
+    const int n = log2L <= 10 ? 1 << log2L : 1024 + (1 << (log2L - 10));
+    for (int t = threadIdx.x; t < n; t += kFftThreads)
+        tl[t] = fft_tw<SIGN>(tw, log2T, (unsigned)(t < 1024 ? t : (t - 1024) << 10) << (log2T - log2L));
+}
+__device__ __forceinline__ float2 stage_tw(const float2* __restrict__ tl, unsigned e) {
+    return e < 1024u ? tl[e] : cmul(tl[e & 1023u], tl[1024 + (e >> 10)]);
 }
 
 // One radix-R Stockham stage over L = 2^log2L points of B = 2^log2B
@@ -70,8 +78,7 @@ __device__ __forceinline__ float2 stage_tw(const float2* __restrict__ tl, const 
 // V = DFT_R(v), out[(j - k) R + k + m Ns] = V_m.
 template <int R, int SIGN>
 __device__ __forceinline__ void smem_stage(const float2* __restrict__ in, float2* __restrict__ out, int log2L,
-                                           int log2B, int log2Ns, const float2* __restrict__ tl,
-                                           const float2* __restrict__ th) {
+                                           int log2B, int log2Ns, const float2* __restrict__ tl) {
     constexpr int LR = ilog2c(R);
     const int B = 1 << log2B;
     const int Lr = 1 << (log2L - LR);
@@ -85,18 +92,20 @@ __device__ __forceinline__ void smem_stage(const float2* __restrict__ in, float2
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = in[((j + r * Lr) << log2B) + cc];
         if (k > 0) {
-            // w^r: powers of two from the tables, the others as products of at most
-            // four of them (15 lookups of a radix-16 task kept the load unit busy)
-            float2 w[R];
+            // w^1, 2, 3 and the multiples of w^4 from the table, the others as one product
+            // (15 lookups of a radix-16 task kept the load unit busy)
+            float2 w[4];
 #pragma unroll
-            for (int r = 1; r < R; r++) {
-                constexpr int top = R;
-                int hb = 1;
-#pragma unroll
-                for (int q = 1; q < top; q *= 2)
-                    if (q <= r) hb = q;
-                w[r] = hb == r ? stage_tw(tl, th, (unsigned)(r * k) << shift) : cmul(w[hb], w[r - hb]);
+            for (int r = 1; r < (R < 4 ? R : 4); r++) {
+                w[r] = stage_tw(tl, (unsigned)(r * k) << shift);
                 v[r] = cmul(v[r], w[r]);
+            }
+#pragma unroll
+            for (int r4 = 4; r4 < R; r4 += 4) {
+                const float2 w4 = stage_tw(tl, (unsigned)(r4 * k) << shift);
+                v[r4] = cmul(v[r4], w4);
+#pragma unroll
+                for (int r = 1; r < 4; r++) v[r4 + r] = cmul(v[r4 + r], cmul(w4, w[r]));
             }
         }
         fft_reg<R, SIGN>(v);
@@ -109,16 +118,15 @@ __device__ __forceinline__ void smem_stage(const float2* __restrict__ in, float2
 // All stages of an L-point FFT on the tile in `a` (natural order in and
 // out); returns the buffer that holds the result.
 template <int SIGN>
-__device__ __forceinline__ float2* smem_fft(float2* a, float2* b, int log2L, int log2B, const float2* __restrict__ tl,
-                                            const float2* __restrict__ th) {
+__device__ __forceinline__ float2* smem_fft(float2* a, float2* b, int log2L, int log2B, const float2* __restrict__ tl) {
     int log2Ns = 0;
     while (log2Ns < log2L) {
         const int lr = min(4, log2L - log2Ns);
         switch (lr) {
-            case 4: smem_stage<16, SIGN>(a, b, log2L, log2B, log2Ns, tl, th); break;
-            case 3: smem_stage<8, SIGN>(a, b, log2L, log2B, log2Ns, tl, th); break;
-            case 2: smem_stage<4, SIGN>(a, b, log2L, log2B, log2Ns, tl, th); break;
-            default: smem_stage<2, SIGN>(a, b, log2L, log2B, log2Ns, tl, th); break;
+            case 4: smem_stage<16, SIGN>(a, b, log2L, log2B, log2Ns, tl); break;
+            case 3: smem_stage<8, SIGN>(a, b, log2L, log2B, log2Ns, tl); break;
+            case 2: smem_stage<4, SIGN>(a, b, log2L, log2B, log2Ns, tl); break;
+            default: smem_stage<2, SIGN>(a, b, log2L, log2B, log2Ns, tl); break;
         }
         __syncthreads();
         float2* s = a;
@@ -143,7 +151,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
                                                           int dst_sel, int log2C, int log2L, int log2B, int mode,
                                                           int r2c, const float2* __restrict__ tw, int log2T) {
     extern __shared__ float2 fft_sm[];
-    __shared__ float2 tl[64], th[64];
+    __shared__ float2 tl[kStageTw];
     const FwdJob J = jobs ? jobs[blockIdx.y] : one;
     const int L = 1 << log2L;
     const int B = 1 << log2B;
@@ -153,11 +161,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
     float2* a = fft_sm;
     float2* b = fft_sm + tot;
     const float2* src = src_sel == 1 ? J.X : J.tmp;
-    // stage twiddles w_L^{SIGN j}: tl for j < 64, th for multiples of 64
-    for (int t = threadIdx.x; t < 128; t += kFftThreads) {
-        const unsigned e = t < 64 ? (unsigned)t : (unsigned)(t - 64) << 6;
-        if (e < (unsigned)L) (t < 64 ? tl[t] : th[t - 64]) = fft_tw<SIGN>(tw, log2T, e << (log2T - log2L));
-    }
+    stage_tw_fill<SIGN>(tl, tw, log2T, log2L);
     for (int t = threadIdx.x; t < tot; t += kFftThreads) {
         int i, cc;
         if (mode == 0) {
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
         a[(i << log2B) + cc] = src_sel == 0 ? fwd_input(J.in_r, J.in_c, J.gain, J.n, j, r2c) : src[j];
     }
     __syncthreads();
-    const float2* res = smem_fft<SIGN>(a, b, log2L, log2B, tl, th);
+    const float2* res = smem_fft<SIGN>(a, b, log2L, log2B, tl);
     float2* dst = dst_sel == 1 ? J.X : J.tmp;
     // inter-pass twiddle w_C^{SIGN col k}: a thread's column is fixed and its k goes up
     // by 128 / B, so the twiddle advances by a factor; looked up again every four
@@ -213,7 +217,7 @@ __global__ void __launch_bounds__(kFftThreads)
                    float cb, float amp, float inv_sigma, float2* __restrict__ H, double* __restrict__ acc_sigma,
                    double* __restrict__ acc_f) {
     extern __shared__ float2 fft_sm[];
-    __shared__ float2 tl[64], th[64];
+    __shared__ float2 tl[kStageTw];
     __shared__ float s_red[kFftThreads / 32][2];
     const int L = 1 << log2L, B = 1 << log2B;
     const int log2S = log2C - log2L;
@@ -224,10 +228,7 @@ __global__ void __launch_bounds__(kFftThreads)
     const int r0 = blockIdx.z * rows_per_cta;
     const int nr = min(rows_per_cta, rows_total - r0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = threadIdx.x; t < 128; t += kFftThreads) {
-        const unsigned e = t < 64 ? (unsigned)t : (unsigned)(t - 64) << 6;
-        if (e < (unsigned)L) (t < 64 ? tl[t] : th[t - 64]) = fft_tw<-1>(tw, log2C, e << (log2C - log2L));
-    }
+    stage_tw_fill<-1>(tl, tw, log2C, log2L);
     float2 h[kAdjColPos], xq[kAdjColPos];
 #pragma unroll
     for (int i = 0; i < kAdjColPos; i++) {
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(kFftThreads)
         __syncthreads();
         for (int t = threadIdx.x; t < tot; t += kFftThreads) a[((t & (L - 1)) << log2B) + (t >> log2L)] = __ldcg(src + t);
         __syncthreads();
-        const float2* res = smem_fft<-1>(a, fft_sm + tot, log2L, log2B, tl, th);
+        const float2* res = smem_fft<-1>(a, fft_sm + tot, log2L, log2B, tl);
         const float2 rc = __ldg(rowc + r0 + r);  // (ca, dfdq)
         float ds = 0.0f, df = 0.0f;
 #pragma unroll

@@ -28,12 +28,17 @@ namespace fcwt {
 constexpr int kP2 = 1024;          // phase-2 transform length
 constexpr int kLog2P2 = 10;
 constexpr int kMaxLog2N = 23;      // N <= 8M samples
-constexpr int kMaxFusedN = 8192;   // rows of N <= this run whole inside one CTA
+constexpr int kMaxFusedN = 8192;   // rows of N <= this run whole inside one CTA (fcwt_small.cu)
 constexpr int kThreads = 256;      // threads per CTA of the row engine (2 CTAs per SM)
 constexpr int kChunk = 64;         // phase-1 k2 values per work item
 constexpr int kMaxK = 32;          // phase-1 transform length held in registers
 constexpr int kGroupCols = 8;      // phase-2 columns per work item (one per warp)
 constexpr int kMaxOuts = 1024;     // output buffers per launch
+
+// Entries of the twiddle table of N: w_N^j for j < 1024, w_N^{1024 j} for j < max(N /
+// 1024, 1), and for 1024 < N <= 8192 all w_N^j (whole rows read single factors there:
+// with products of two in the stages the error was 2.5e-7 instead of 1.9e-7).
+constexpr int tw_entries(int N) { return 1024 + (N >= 1024 ? N / 1024 : 1) + (N > 1024 && N <= 8192 ? N : 0); }
 
 // One input signal of a launch (a batch may hold several).
 struct SigDesc {
@@ -76,7 +81,7 @@ struct RowDesc {
     int n_out;        // output samples of the row: ceil(n / D)
 };
 
-enum ItemType : int { ITEM_FUSED = 0, ITEM_PHASE1 = 1, ITEM_PHASE2 = 2, ITEM_SMALL = 3, ITEM_PHASE1W = 4 };
+enum ItemType : int { ITEM_PHASE1 = 1, ITEM_PHASE2 = 2, ITEM_PHASE1W = 4 };
 
 // Rows whose window needs K > kMaxK use warp-cooperative phase-1 items: each
 // covers kWideChunk consecutive k2 (one per warp) for all v.
@@ -113,6 +118,11 @@ __host__ __device__ inline int perm_bin(int q, int log2R) {
 }
 
 // Everything the row engine needs for one launch.
+// Output buffers of a launch, one per signal.
+struct OutPtrs {
+    void* p[kMaxOuts];
+};
+
 struct EngineParams {
     const SigDesc* sigs;
     const RowDesc* rows;

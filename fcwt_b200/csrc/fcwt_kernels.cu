@@ -37,14 +37,14 @@ __global__ void k_mother(float fb, int N, float norm, float* __restrict__ out) {
     out[w] = __fmul_rn(norm, e);
 }
 
-// tw[j] = w_N^j for j < 1024; tw[1024 + j] = w_N^{1024 j} for j < max(M, 1).
-// w_N = exp(+2 pi i / N).
+// tw[j] = w_N^j for j < 1024; tw[1024 + j] = w_N^{1024 j} for j < max(M, 1);
+// tw[1024 + M + j] = w_N^j for all j when 1024 < N <= 8192. w_N = exp(+2 pi i / N).
 __global__ void k_twiddle(int log2N, float2* __restrict__ tw) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = 1 << log2N;
     const int M = N >= 1024 ? N / 1024 : 1;
-    if (j >= 1024 + M) return;
-    long long e = j < 1024 ? j : (long long)(j - 1024) * 1024;
+    if (j >= tw_entries(N)) return;
+    long long e = j < 1024 ? j : j < 1024 + M ? (long long)(j - 1024) * 1024 : j - 1024 - M;
     e &= (long long)N - 1;
     double s, c;
     sincospi(2.0 * (double)e / (double)N, &s, &c);
@@ -54,7 +54,7 @@ __global__ void k_twiddle(int log2N, float2* __restrict__ tw) {
 // --------------------------------------------------------------- row engine
 
 // Shared-memory layout of the row engine, per CTA (units of float2):
-//   region0: G of a fused row (<= 8192) / per-warp transposes (8 x 32x33) /
+//   region0: per-warp transposes (8 x 32x33) /
 //            output staging [1024][9] of 8 columns
 //   zs:      phase-1 input tile [K][kChunk]
 //   twlo:    w_N^j, j < 1024, of the current N
@@ -71,7 +71,6 @@ constexpr size_t kSmemAlign = 1024;  // the 64B-swizzled staging tile wants 1 KB
 constexpr size_t kEngineSmemBytes = (size_t)kSmemFloat2 * sizeof(float2) + kSmemAlign;
 static_assert(4 * kBoxBytes <= kRegion0 * 8, "staging boxes fit in region0");
 constexpr int kFetchBatch = 2;  // work items claimed per queue access
-static_assert(kRegion0 >= kMaxFusedN, "fused rows keep G in region0");
 static_assert(kRegion0 >= (kThreads / 32) * 32 * 33, "per-warp transposes live in region0");
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -120,7 +119,7 @@ __device__ __forceinline__ float2 tw_n(const float2* __restrict__ twlo, const Tw
 // Phase 1 of one chunk of kChunk k2 values of a row (see fcwt_internal.h):
 // loads Z into the tile zs[k1][k2], then every (k2, v) task runs a K-point
 // DFT and writes G[c][k2] (c = v + R u) times w_N^{(k2+L) c}.
-template <int K, bool TO_GLOBAL>
+template <int K>
 __device__ __forceinline__ void phase1_chunk(const SigDesc& S, const RowDesc& R, const float* __restrict__ pool, int k2_0,
                              float2* __restrict__ zs, const float2* __restrict__ twlo,
                              const TwM twhi, float2* __restrict__ gdst) {
@@ -176,27 +175,23 @@ __device__ __forceinline__ void phase1_chunk(const SigDesc& S, const RowDesc& R,
             w = (u & 7) ? cmul(w, wd) : tw_n(twlo, twhi, eu & Nm);
             eu += d;
             const float2 g = cmul(z[u], w);
-            if constexpr (TO_GLOBAL)
-                __stcg(p, g);
-            else
-                *p = g;
+            __stcg(p, g);
             p += pstep;
         }
     }
     __syncthreads();
 }
 
-template <bool TO_GLOBAL>
 __device__ void phase1_chunk_dispatch(int K, const SigDesc& S, const RowDesc& R, const float* pool,
                                       int k2_0, float2* zs, const float2* twlo, const TwM twhi,
                                       float2* gdst) {
     switch (K) {
-        case 1: phase1_chunk<1, TO_GLOBAL>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
-        case 2: phase1_chunk<2, TO_GLOBAL>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
-        case 4: phase1_chunk<4, TO_GLOBAL>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
-        case 8: phase1_chunk<8, TO_GLOBAL>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
-        case 16: phase1_chunk<16, TO_GLOBAL>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
-        default: phase1_chunk<32, TO_GLOBAL>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
+        case 1: phase1_chunk<1>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
+        case 2: phase1_chunk<2>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
+        case 4: phase1_chunk<4>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
+        case 8: phase1_chunk<8>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
+        case 16: phase1_chunk<16>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
+        default: phase1_chunk<32>(S, R, pool, k2_0, zs, twlo, twhi, gdst); break;
     }
 }
 
@@ -530,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         const TwM twhi = Mcols <= kTwhiSmem ? TwM{twhi_s, nullptr} : TwM{twhi_s, twhi_s + 32};
 
         // region0 may still be read by the bulk stores of the previous phase-2 item
-        if (P.tma_store && (item.type == ITEM_PHASE2 || item.type == ITEM_FUSED || item.type == ITEM_PHASE1W)) {
+        if (P.tma_store && (item.type == ITEM_PHASE2 || item.type == ITEM_PHASE1W)) {
             if (tid == 0) bulk_wait_read_all();
             __syncthreads();
         }
@@ -547,50 +542,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             if (tid == 0) s_log2N = log2N;
         }
 
-        if (item.type == ITEM_SMALL) {
-            // N < 1024: direct DFT over the row's nonzero bins.
-            const int lo = R.lo, hi = R.hi;
-            const float nm1 = (float)N - 1.0f;
-            for (int q = lo + tid; q < hi; q += kThreads) zs[q - lo] = bin_value(R, S, P.stale_pool, nm1, q);
-            __syncthreads();
-            for (int to = tid; to < R.n_out; to += kThreads) {
-                const int t = to * R.dec;
-                float2 acc = make_float2(0.0f, 0.0f);
-                for (int q = lo; q < hi; q++) {
-                    const float2 w = twlo[(q * t) & (N - 1)];
-                    const float2 z = zs[q - lo];
-                    acc.x += z.x * w.x - z.y * w.y;
-                    acc.y += z.x * w.y + z.y * w.x;
-                }
-                store_out<OT>(outb, R.out_off + to, acc);
-            }
-        } else if (item.type == ITEM_FUSED) {
-            // whole row in this CTA (N <= 8192, M <= 8 columns): phase 1 into
-            // SMEM, then one warp per column
-            const int M = N >> kLog2P2;
-            for (int k2_0 = 0; k2_0 < kP2; k2_0 += kChunk)
-                phase1_chunk_dispatch<false>(R.K, S, R, P.stale_pool, k2_0, zs, twlo, twhi, region0);
-            float2 x[32];
-            if (warp < M) {
-#pragma unroll
-                for (int m = 0; m < 32; m++) x[m] = region0[warp * kP2 + lane + 32 * m];
-            }
-            __syncthreads();
-            if (warp < M) dft1024_warp(x, lane, region0 + warp * (32 * 33), t2);
-            __syncthreads();
-            if (warp < M) {
-#pragma unroll
-                for (int h = 0; h < 32; h++) region0[(lane + 32 * h) * kStagePitch + warp] = x[h];
-            }
-            __syncthreads();
-            const int log2M = log2N - kLog2P2;
-            for (int to = tid; to < R.n_out; to += kThreads) {
-                const int t = to * R.dec;
-                const int c = t & (M - 1);
-                const int a = t >> log2M;
-                store_out<OT>(outb, R.out_off + to, region0[a * kStagePitch + c]);
-            }
-        } else if (item.type == ITEM_PHASE1) {
+        if (item.type == ITEM_PHASE1) {
             if (tid == 0) {
                 s_ok = 1;
                 if (R.wait_row >= 0)
@@ -599,7 +551,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             __syncthreads();
             if (s_ok) {
                 float2* G = P.scratch + (size_t)R.slot * (size_t)P.slot_elems;
-                phase1_chunk_dispatch<true>(R.K, S, R, P.stale_pool, item.part * kChunk, zs, twlo, twhi, G);
+                phase1_chunk_dispatch(R.K, S, R, P.stale_pool, item.part * kChunk, zs, twlo, twhi, G);
                 if (tid == 0) {
                     __threadfence();
                     red_release_add(a_done + item.row, 1u);
@@ -655,8 +607,7 @@ cudaError_t launch_mother(float fb, int N, float norm, float* out, cudaStream_t 
 
 cudaError_t launch_twiddle(int log2N, float2* tw, cudaStream_t st) {
     const int N = 1 << log2N;
-    const int M = N >= 1024 ? N / 1024 : 1;
-    const int total = 1024 + M;
+    const int total = tw_entries(N);
     dev::k_twiddle<<<(total + 255) / 256, 256, 0, st>>>(log2N, tw);
     return cudaGetLastError();
 }

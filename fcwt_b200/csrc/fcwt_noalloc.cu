@@ -46,6 +46,9 @@ cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log
 cudaError_t engine_configure();
 cudaError_t engine_blocks_per_sm(int* out);
 cudaError_t launch_engine(const EngineParams& p, int grid, cudaStream_t st);
+cudaError_t small_configure();
+cudaError_t launch_rows_small(const SigDesc* sigs, const RowDesc* rows, const int* list, int n_list, const float* pool,
+                              const OutPtrs& outs, int out_type, int log2L, cudaStream_t st);
 void record_error(const std::string& msg);  // message returned by fcwt_last_error()
 }  // namespace fcwt
 
@@ -65,7 +68,8 @@ constexpr size_t kOffX = 0;
 constexpr size_t kOffTmp = align256(kOffX + sizeof(float2) * kNaMaxN);
 constexpr size_t kOffMother = align256(kOffTmp + sizeof(float2) * kNaMaxN);
 constexpr size_t kOffTw = align256(kOffMother + sizeof(float) * kNaMaxN);
-constexpr size_t kOffPool = align256(kOffTw + sizeof(float2) * (kP2 + kNaMaxN / kP2));
+static_assert(tw_entries(kMaxFusedN) >= tw_entries(kNaMaxN), "the table of N <= 8192 is the largest");
+constexpr size_t kOffPool = align256(kOffTw + sizeof(float2) * tw_entries(kMaxFusedN));
 constexpr size_t kOffRows = align256(kOffPool + sizeof(float) * kNaMaxTables * (kNaMaxN / 2));
 constexpr size_t kOffItems = align256(kOffRows + sizeof(RowDesc) * kNaMaxRows);
 constexpr size_t kOffSig = align256(kOffItems + sizeof(Item) * kNaMaxItems);
@@ -108,15 +112,10 @@ __global__ void k_na_pool(const __grid_constant__ PoolCopy c, float* __restrict_
 }
 
 // The work list of the row engine, the same sequence the host builds for a
-// plan: one item per row when rows run whole (type), otherwise per step s,
-// the n_a phase-1 items of row s (s < fn) followed by the n_b phase-2 items of
-// row s - lag (0 <= s - lag < fn). One thread per step.
-__global__ void k_na_items(int fn, int two_phase, int type, int n_a, int n_b, int lag, Item* __restrict__ items) {
+// plan: per step s, the n_a phase-1 items of row s (s < fn) followed by the n_b
+// phase-2 items of row s - lag (0 <= s - lag < fn). One thread per step.
+__global__ void k_na_items(int fn, int n_a, int n_b, int lag, Item* __restrict__ items) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!two_phase) {
-        if (s < fn) items[s] = Item{type, s, 0, 0};
-        return;
-    }
     if (s >= fn + lag) return;
     int base = n_a * min(s, fn) + n_b * max(0, min(s - lag, fn));
     if (s < fn)
@@ -152,6 +151,7 @@ int setup_device(int dev, DeviceSetup** out) {
         if (e != cudaSuccess)
             return na_fail(FCWT_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
         e = engine_configure();
+        if (e == cudaSuccess) e = small_configure();
         if (e != cudaSuccess) return na_fail(FCWT_ERR_CUDA, std::string("engine set-up: ") + cudaGetErrorString(e));
         int per_sm = 0, sms = 0;
         e = engine_blocks_per_sm(&per_sm);
@@ -255,7 +255,7 @@ extern "C" int fcwt_cwt_noalloc(const float* input, int n, float fb, const float
         d.cb = rp.cb;
         d.cnorm = host::mother_norm();
     }
-    const int n_items = two_phase ? fn * (n_a + n_b) : fn;
+    const int n_items = fn * (n_a + n_b);
 
     unsigned char* base = S->base;
     float2* X = reinterpret_cast<float2*>(base + kOffX);
@@ -302,9 +302,10 @@ extern "C" int fcwt_cwt_noalloc(const float* input, int n, float fb, const float
                 NA_TRY(cudaGetLastError());
             }
         }
-        k_na_items<<<(fn + lag + 127) / 128, 128, 0, st>>>(fn, two_phase ? 1 : 0, N < kP2 ? ITEM_SMALL : ITEM_FUSED,
-                                                             n_a, n_b, lag, ditems);
-        NA_TRY(cudaGetLastError());
+        if (two_phase) {
+            k_na_items<<<(fn + lag + 127) / 128, 128, 0, st>>>(fn, n_a, n_b, lag, ditems);
+            NA_TRY(cudaGetLastError());
+        }
     }
     NA_TRY(cudaMemsetAsync(counters, 0, sizeof(unsigned) * (1 + 2 * (size_t)fn), st));
     NA_TRY(cudaMemsetAsync(derr, 0, sizeof(int), st));
@@ -312,21 +313,28 @@ extern "C" int fcwt_cwt_noalloc(const float* input, int n, float fb, const float
     NA_TRY(launch_twiddle(sp.log2N, tw, st));
     int n_fwd = 0;
     NA_TRY(launch_forward(input, nullptr, n, sp.log2N, tw, X, tmp, st, &n_fwd, nullptr, 0));
-    EngineParams ep;
-    std::memset(&ep, 0, sizeof(ep));
-    ep.sigs = dsig;
-    ep.rows = drows;
-    ep.items = ditems;
-    ep.n_items = n_items;
-    ep.stale_pool = dpool;
-    ep.scratch = two_phase ? scratch : nullptr;
-    ep.slot_elems = two_phase ? N : 0;
-    ep.counters = counters;
-    ep.n_rows = fn;
-    ep.outs[0] = output;
-    ep.out_type = OUT_C64;
-    ep.err = derr;
-    NA_TRY(launch_engine(ep, std::max(1, std::min(ep.n_items, S->grid)), st));
+    if (two_phase) {
+        EngineParams ep;
+        std::memset(&ep, 0, sizeof(ep));
+        ep.sigs = dsig;
+        ep.rows = drows;
+        ep.items = ditems;
+        ep.n_items = n_items;
+        ep.stale_pool = dpool;
+        ep.scratch = scratch;
+        ep.slot_elems = N;
+        ep.counters = counters;
+        ep.n_rows = fn;
+        ep.outs[0] = output;
+        ep.out_type = OUT_C64;
+        ep.err = derr;
+        NA_TRY(launch_engine(ep, std::max(1, std::min(ep.n_items, S->grid)), st));
+    } else {
+        OutPtrs outs;
+        std::memset(&outs, 0, sizeof(outs));
+        outs.p[0] = output;
+        NA_TRY(launch_rows_small(dsig, drows, nullptr, fn, dpool, outs, OUT_C64, sp.log2N, st));
+    }
     if (status) {
         int h = 0;
         NA_TRY(cudaMemcpyAsync(&h, derr, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -295,3 +295,30 @@ def test_tensor_core_tiling_edges(fcwt, oracle, n, dec, f1):
     ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)[:, ::dec]
     for r in range(fn):
         assert rel_l2(got[r], ref[r]) <= 3.3e-6, r
+
+
+@pytest.mark.parametrize("n,dec,cplx", [
+    (1, 1, False), (2, 1, True), (3, 1, False), (17, 1, True), (33, 32, False), (1000, 1, False), (1024, 4, True),
+    (1025, 1, False), (2048, 2048, False), (4095, 1, True), (4097, 2, False), (8191, 64, False), (8192, 1, True),
+])
+def test_whole_row_sizes(fcwt, oracle, n, dec, cplx):
+    """Rows of one CTA at the smallest, largest and odd lengths, decimated up to a
+    single sample. Bound: two transforms of at most 13 butterfly levels and 4
+    twiddles each, 2^-24 per rounding of a level and 2^-22 per twiddle:
+    26 x 2^-24 + 8 x 2^-22 = 3.5e-6 if all were to add up."""
+    import torch
+
+    fn = 7
+    sc = fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LOGSCALES, 1000, 20, 450, fn)
+    rng = np.random.default_rng(n + dec)
+    x = rng.standard_normal(n).astype(np.float32)
+    if cplx:
+        x = (x + 1j * rng.standard_normal(n)).astype(np.complex64)
+    plan = fcwt.Plan(n, sc, fb=2.0, complex_input=cplx, time_stride=dec)
+    out = torch.full(plan.out_shape, float("nan"), dtype=torch.complex64, device="cuda")
+    plan.execute(torch.from_numpy(x).cuda(), out)
+    got = out.cpu().numpy()
+    plan.close()
+    ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)[:, ::dec]
+    for r in range(fn):
+        assert np.linalg.norm(got[r] - ref[r]) <= 3.5e-6 * np.linalg.norm(ref[r]) + 1e-30, r
