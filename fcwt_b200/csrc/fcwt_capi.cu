@@ -28,9 +28,10 @@ size_t engine_smem_bytes();
 cudaError_t launch_mother(float fb, int N, float norm, float* out, cudaStream_t st);
 cudaError_t launch_twiddle(int log2N, float2* tw, cudaStream_t st);
 cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log2N, const float2* tw,
-                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R);
+                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R,
+                           unsigned* zero = nullptr, int n_zero = 0);
 cudaError_t launch_forward_batched(const FwdJob* jobs, int njobs, int log2N, const float2* tw, cudaStream_t st,
-                                   int* n_kernels, bool real);
+                                   int* n_kernels, bool real, unsigned* zero = nullptr, int n_zero = 0);
 cudaError_t launch_inverse_batched(const FwdJob* jobs, int njobs, int log2N, const float2* tw, cudaStream_t st,
                                    int* n_kernels);
 cudaError_t launch_adjoint_accum(const float2* Xs, const float2* Gh, float2* H, const void* rows, int nr, int half,
@@ -750,6 +751,13 @@ int plan_build(fcwt_plan* P) {
     return FCWT_OK;
 }
 
+// The error word of the finished executions, cleared for the next ones.
+int take_engine_error(fcwt_context* ctx) {
+    const int bits = *ctx->err_host;
+    *ctx->err_host = 0;
+    return bits ? fail(FCWT_ERR_DEVICE, "row engine reported error bits " + std::to_string(bits)) : FCWT_OK;
+}
+
 // Queue counters of one execution: [0] item queue; a_done[rows]; b_done[rows];
 // two tensor-core row queues.
 size_t plan_counters(const fcwt_plan* P) { return 3 + 2 * (size_t)P->n_rows; }
@@ -811,8 +819,8 @@ void build_jobs(fcwt_plan* P, const void* const* din, std::vector<std::pair<int,
     job_groups(P, groups);
 }
 
-int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type);
-int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* graph_jobs);
+int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type, int* err);
+int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* graph_jobs, unsigned* zero, int n_zero);
 
 // Enqueues the forward FFTs and the row engine for device-resident inputs and
 // outputs (no host synchronisation, so it can be captured into a graph).
@@ -826,10 +834,21 @@ int plan_enqueue(fcwt_plan* P, const void* const* din, void* const* dout, int ou
         return fail(FCWT_ERR_UNSUPPORTED, "doublesided wavelets write complex64 outputs only");
     if (P->compat_align && out_type != FCWT_OUT_C64)
         return fail(FCWT_ERR_UNSUPPORTED, "FCWT_COMPAT_ALIGN writes complex64 outputs only");
-    int rc = enqueue_forward(P, din, graph_jobs);
+    // The counters are cleared by the first forward kernel. The engine with waits between
+    // CTAs polls its error word, so that word is in device memory, cleared and copied
+    // back; the others only write theirs, when a wait runs out: they are given the host's
+    // word itself. (Two memsets, a copy of 4 bytes and the split kernel were 11 of the 26
+    // us of a 1000 x 64 call.)
+    const size_t n_counters = plan_counters(P);
+    FCWT_CUDA_TRY(ctx->counters.ensure(n_counters * sizeof(unsigned)));
+    int rc = enqueue_forward(P, din, graph_jobs, ctx->counters.as<unsigned>(), (int)n_counters);
     if (rc) return rc;
-    FCWT_CUDA_TRY(ctx->err.ensure(sizeof(int)));
-    FCWT_CUDA_TRY(cudaMemsetAsync(ctx->err.p, 0, sizeof(int), st));
+    int* err = ctx->err_host;
+    if (P->n_items > 0) {
+        FCWT_CUDA_TRY(ctx->err.ensure(sizeof(int)));
+        FCWT_CUDA_TRY(cudaMemsetAsync(ctx->err.p, 0, sizeof(int), st));
+        err = ctx->err.as<int>();
+    }
     std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
     const bool prof = ctx->profiling && allow_profiling;
     if (prof) {
@@ -842,7 +861,7 @@ int plan_enqueue(fcwt_plan* P, const void* const* din, void* const* dout, int ou
         }
         FCWT_CUDA_TRY(cudaEventRecord(ev.first, st));
     }
-    rc = enqueue_rows(P, P->sigs.as<SigDesc>(), dout, out_type);
+    rc = enqueue_rows(P, P->sigs.as<SigDesc>(), dout, out_type, err);
     if (rc) return rc;
     if (P->doublesided) {
         // the mirrored half: exp(-2 pi i t / N) conj(V), V the rows on the shifted spectrum
@@ -851,7 +870,8 @@ int plan_enqueue(fcwt_plan* P, const void* const* din, void* const* dout, int ou
         FCWT_CUDA_TRY(launch_shift_spectrum(S.X.as<float2>(), S.sp.log2N, P->Xs.as<float2>(),
                                             S.log2R ? P->Xsp.as<float2>() : nullptr, S.log2R, st));
         void* tmp_out[1] = {P->ds_tmp.p};
-        rc = enqueue_rows(P, P->sigs2.as<SigDesc>(), tmp_out, out_type);
+        FCWT_CUDA_TRY(cudaMemsetAsync(ctx->counters.p, 0, n_counters * sizeof(unsigned), st));
+        rc = enqueue_rows(P, P->sigs2.as<SigDesc>(), tmp_out, out_type, err);
         if (rc) return rc;
         FCWT_CUDA_TRY(launch_doublesided_combine(static_cast<float2*>(dout[0]), P->ds_tmp.as<float2>(),
                                                  S.rows_out(), S.n_out(), S.dec, S.sp.log2N, tw,
@@ -872,12 +892,14 @@ int plan_enqueue(fcwt_plan* P, const void* const* din, void* const* dout, int ou
         FCWT_CUDA_TRY(cudaEventRecord(ev.second, st));
         ctx->ev_used.push_back(ev);
     }
-    FCWT_CUDA_TRY(cudaMemcpyAsync(ctx->err_host, ctx->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (P->n_items > 0)
+        FCWT_CUDA_TRY(cudaMemcpyAsync(ctx->err_host, ctx->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     return FCWT_OK;
 }
 
-// The forward FFTs of all signals of a plan into their spectra.
-int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* graph_jobs) {
+// The forward FFTs of all signals of a plan into their spectra; the first kernel
+// also clears the n_zero queue counters at `zero`.
+int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* graph_jobs, unsigned* zero, int n_zero) {
     using namespace fcwt;
     fcwt_context* ctx = P->ctx;
     cudaStream_t st = ctx->stream;
@@ -890,7 +912,7 @@ int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* gr
                                      S.sp.is_complex ? (const float2*)din[0] : nullptr, S.sp.n, S.sp.log2N,
                                      P->tables[(size_t)S.table].tw.as<float2>(), S.X.as<float2>(),
                                      ctx->tmp.as<float2>(), st, &n_fwd, S.log2R ? S.Xp.as<float2>() : nullptr,
-                                     S.log2R));
+                                     S.log2R, zero, n_zero));
         ctx->kernel_launches += n_fwd;
     } else {
         // batched forward FFTs, one launch sequence per padded length
@@ -914,7 +936,7 @@ int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* gr
             int n_fwd = 0;
             FCWT_CUDA_TRY(launch_forward_batched(djobs + off, g.second, P->tables[(size_t)g.first].log2N,
                                                  P->tables[(size_t)g.first].tw.as<float2>(), st, &n_fwd,
-                                                 !P->is_complex));
+                                                 !P->is_complex, off == 0 ? zero : nullptr, off == 0 ? n_zero : 0));
             ctx->kernel_launches += n_fwd;
             off += g.second;
         }
@@ -924,14 +946,12 @@ int enqueue_forward(fcwt_plan* P, const void* const* din, const fcwt::FwdJob* gr
 
 // The row-engine launches of one pass over the plan's rows, reading the
 // spectra of `dsigs` and writing `dout`.
-int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type) {
+int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, int out_type, int* err) {
     using namespace fcwt;
     fcwt_context* ctx = P->ctx;
     cudaStream_t st = ctx->stream;
     const int nsig = (int)P->sig.size();
     const size_t n_counters = plan_counters(P);
-    FCWT_CUDA_TRY(ctx->counters.ensure(n_counters * sizeof(unsigned)));
-    FCWT_CUDA_TRY(cudaMemsetAsync(ctx->counters.p, 0, n_counters * sizeof(unsigned), st));
     if (P->two_phase)
         FCWT_CUDA_TRY(ctx->scratch.ensure((size_t)P->slots * (size_t)P->slot_elems * sizeof(float2)));
     EngineParams ep;
@@ -947,7 +967,7 @@ int enqueue_rows(fcwt_plan* P, const fcwt::SigDesc* dsigs, void* const* dout, in
     ep.n_rows = P->n_rows;
     for (int s = 0; s < nsig; s++) ep.outs[s] = dout[s];
     ep.out_type = out_type;
-    ep.err = ctx->err.as<int>();
+    ep.err = err;
     CUtensorMap omap;
     std::memset(&omap, 0, sizeof(omap));
     int map_ok = 0;
@@ -1023,12 +1043,9 @@ int run_pipelined(fcwt_plan* P, const void* din, void* hout, int out_type) {
             FCWT_CUDA_TRY(cudaEventCreateWithFlags(&ctx->pipe_copied[i], cudaEventDisableTiming));
     }
     const void* din_arr[1] = {din};
-    int rc = enqueue_forward(P, din_arr, nullptr);
-    if (rc) return rc;
-    FCWT_CUDA_TRY(ctx->err.ensure(sizeof(int)));
-    FCWT_CUDA_TRY(cudaMemsetAsync(ctx->err.p, 0, sizeof(int), st));
     FCWT_CUDA_TRY(ctx->counters.ensure((size_t)nblk * sizeof(unsigned)));
-    FCWT_CUDA_TRY(cudaMemsetAsync(ctx->counters.p, 0, (size_t)nblk * sizeof(unsigned), st));
+    int rc = enqueue_forward(P, din_arr, nullptr, ctx->counters.as<unsigned>(), nblk);
+    if (rc) return rc;
     std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
     const bool prof = ctx->profiling;
     if (prof) {
@@ -1061,7 +1078,7 @@ int run_pipelined(fcwt_plan* P, const void* din, void* hout, int out_type) {
         tp.atab = P->tc_tabs.as<unsigned char>();
         tp.counter = ctx->counters.as<unsigned>() + b;
         tp.outs[0] = base;
-        tp.err = ctx->err.as<int>();
+        tp.err = ctx->err_host;
         FCWT_CUDA_TRY(launch_tc(tp, S.log2R, out_type, std::max(1, std::min(r1 - r0, ctx->num_sms)), st));
         ctx->kernel_launches += 1;
         FCWT_CUDA_TRY(cudaEventRecord(ctx->pipe_done[slot], st));
@@ -1074,12 +1091,9 @@ int run_pipelined(fcwt_plan* P, const void* din, void* hout, int out_type) {
         FCWT_CUDA_TRY(cudaEventRecord(ev.second, st));
         ctx->ev_used.push_back(ev);
     }
-    FCWT_CUDA_TRY(cudaMemcpyAsync(ctx->err_host, ctx->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     FCWT_CUDA_TRY(cudaStreamSynchronize(ctx->copy_stream));
     FCWT_CUDA_TRY(cudaStreamSynchronize(st));
-    if (*ctx->err_host != 0)
-        return fail(FCWT_ERR_DEVICE, "row engine reported error bits " + std::to_string(*ctx->err_host));
-    return FCWT_OK;
+    return take_engine_error(ctx);
 }
 
 // Runs a plan on host or device buffers: host inputs are staged in, host
@@ -1149,8 +1163,7 @@ int plan_run_multi(fcwt_plan* P, const void* const* inputs, void* const* outputs
             if (dout[(size_t)s] != outputs[s] && out_bytes[(size_t)s])
                 FCWT_CUDA_TRY(cudaMemcpyAsync(outputs[s], dout[(size_t)s], out_bytes[(size_t)s], cudaMemcpyDeviceToHost, st));
         FCWT_CUDA_TRY(cudaStreamSynchronize(st));
-        if (*ctx->err_host != 0)
-            return fail(FCWT_ERR_DEVICE, "row engine reported error bits " + std::to_string(*ctx->err_host));
+        return take_engine_error(ctx);
     }
     return FCWT_OK;
 }
@@ -1339,12 +1352,7 @@ int fcwt_synchronize(fcwt_context* ctx) {
     int rc = ctx_prepare(ctx);
     if (rc) return rc;
     FCWT_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (*ctx->err_host != 0) {
-        int bits = *ctx->err_host;
-        *ctx->err_host = 0;
-        return fail(FCWT_ERR_DEVICE, "row engine reported error bits " + std::to_string(bits));
-    }
-    return FCWT_OK;
+    return take_engine_error(ctx);
 }
 
 int fcwt_profile_enable(fcwt_context* ctx, int enable) {

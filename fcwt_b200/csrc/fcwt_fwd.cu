@@ -17,8 +17,8 @@
 // consecutive elements of global memory.
 //
 // A real signal of N = 2C samples is transformed as the C-point FFT of its
-// sample pairs z[j] = x[2j] + i x[2j+1], then split into all N bins
-// (k_r2c_split). Complex inputs and the inverse transforms run the C = N
+// sample pairs z[j] = x[2j] + i x[2j+1], whose last pass splits it into the bins
+// up to N / 2 of the real signal. Complex inputs and the inverse transforms run the C = N
 // complex FFT.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -143,13 +143,27 @@ __device__ __forceinline__ float2* smem_fft(float2* a, float2* b, int log2L, int
 //   mode 0 (pass A): column col holds elements col + S i; its results are
 //                    multiplied by w_C^{SIGN col k};
 //   mode 1 (pass B): column col holds elements col L + i.
-// Result k of column col goes to col + S k in both modes. src/dst: 0 = the
-// job's input (zero padded; r2c: sample pairs), 1 = its spectrum X, 2 = its
-// tmp buffer.
-template <int SIGN>
+// Result k of column col goes to col + S k in both modes. src_sel: 0 = the
+// job's input (zero padded; r2c: sample pairs), 2 = its tmp buffer; dst_sel:
+// 1 = its spectrum X, 2 = its tmp buffer.
+//
+// SPLIT (the last pass of a real input's transform, mode 1): the results are
+// Z = FFT_{N/2}(z) of the sample pairs, and the CTA writes the spectrum itself. With
+// E = (Z[k] + conj Z[N/2-k]) / 2 and O = -i (Z[k] - conj Z[N/2-k]) / 2,
+//   X[k] = E + w_N^{-k} O,   X[N/2 - k] = conj(E - w_N^{-k} O);
+// bins above N / 2 are conjugates that no reader uses. Bin col + S k pairs with
+// bin (S - col) + S (L - 1 - k), so the CTA takes B / 2 columns from
+// B / 2 blockIdx.x on and their partners S - col (column 0, whose bins pair among
+// themselves, comes with column S / 2, whose bins do too). A split kernel of
+// its own cost a call one launch and one pass over the spectrum (with the memsets and
+// the copy that went at the same time: 10000 samples x 200 rows 46 -> 40 us a call).
+//
+// zero: n_zero words to clear for the kernels after the transform.
+template <int SIGN, bool SPLIT>
 __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restrict__ jobs, FwdJob one, int src_sel,
                                                           int dst_sel, int log2C, int log2L, int log2B, int mode,
-                                                          int r2c, const float2* __restrict__ tw, int log2T) {
+                                                          int r2c, const float2* __restrict__ tw, int log2T,
+                                                          unsigned* __restrict__ zero, int n_zero) {
     extern __shared__ float2 fft_sm[];
     __shared__ float2 tl[kStageTw];
     const FwdJob J = jobs ? jobs[blockIdx.y] : one;
@@ -157,10 +171,13 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
     const int B = 1 << log2B;
     const int log2S = log2C - log2L;
     const int tot = L << log2B;
-    const int c0 = blockIdx.x << log2B;
+    const int log2H = SPLIT && log2S > 0 ? log2B - 1 : log2B;  // columns of the CTA's own, without the partners
+    const int c0 = blockIdx.x << log2H;
+    if (zero && blockIdx.x == 0 && blockIdx.y == 0)
+        for (int t = threadIdx.x; t < n_zero; t += kFftThreads) zero[t] = 0;
     float2* a = fft_sm;
     float2* b = fft_sm + tot;
-    const float2* src = src_sel == 1 ? J.X : J.tmp;
+    const float2* src = J.tmp;
     stage_tw_fill<SIGN>(tl, tw, log2T, log2L);
     for (int t = threadIdx.x; t < tot; t += kFftThreads) {
         int i, cc;
@@ -171,12 +188,52 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
             i = t & (L - 1);
             cc = t >> log2L;
         }
-        const int col = c0 + cc;
+        int col = c0 + cc;
+        if (SPLIT && (cc >> log2H)) {
+            const int own = col - (1 << log2H);
+            col = own == 0 ? 1 << (log2S - 1) : (1 << log2S) - own;
+        }
         const int j = mode == 0 ? col + (i << log2S) : (col << log2L) + i;
         a[(i << log2B) + cc] = src_sel == 0 ? fwd_input(J.in_r, J.in_c, J.gain, J.n, j, r2c) : src[j];
     }
     __syncthreads();
     const float2* res = smem_fft<SIGN>(a, b, log2L, log2B, tl);
+    if constexpr (SPLIT) {
+        const int C = 1 << log2C;
+        auto emit = [&](int q, float2 A, float2 Bz) {
+            const float2 E = make_float2(0.5f * (A.x + Bz.x), 0.5f * (A.y - Bz.y));
+            const float2 O = make_float2(0.5f * (A.y + Bz.y), -0.5f * (A.x - Bz.x));
+            const float2 wo = cmul(fft_tw<SIGN>(tw, log2T, (unsigned)q), O);
+            const float2 xk = make_float2(E.x + wo.x, E.y + wo.y);
+            const float2 yk = make_float2(E.x - wo.x, wo.y - E.y);
+            J.X[q] = xk;
+            if (J.log2R) J.Xp[perm_bin(q, J.log2R)] = xk;
+            if (2 * q == C) return;
+            J.X[C - q] = yk;
+            if (J.log2R && q > 0) J.Xp[perm_bin(C - q, J.log2R)] = yk;
+        };
+        if (log2S == 0) {
+            for (int k = threadIdx.x; k <= L / 2; k += kFftThreads) emit(k, res[k], res[(L - k) & (L - 1)]);
+            return;
+        }
+        for (int t = threadIdx.x; t < L << log2H; t += kFftThreads) {
+            const int cc = t & ((1 << log2H) - 1);
+            const int k = t >> log2H;
+            const int col = c0 + cc;
+            const float2* own = res + cc;
+            const float2* par = own + (1 << log2H);
+            if (col > 0) {
+                emit(col + (k << log2S), own[k << log2B], par[(L - 1 - k) << log2B]);
+            } else if (k < L / 2) {
+                emit(k << log2S, own[k << log2B], own[((L - k) & (L - 1)) << log2B]);
+            } else {
+                const int k2 = k - L / 2;
+                emit((1 << (log2S - 1)) + (k2 << log2S), par[k2 << log2B], par[(L - 1 - k2) << log2B]);
+                if (k2 == 0) emit(C / 2, own[(L / 2) << log2B], own[(L / 2) << log2B]);
+            }
+        }
+        return;
+    }
     float2* dst = dst_sel == 1 ? J.X : J.tmp;
     // inter-pass twiddle w_C^{SIGN col k}: a thread's column is fixed and its k goes up
     // by 128 / B, so the twiddle advances by a factor; looked up again every four
@@ -295,58 +352,27 @@ __global__ void __launch_bounds__(kFftThreads)
     }
 }
 
-// Real-input split: with Z = FFT_{N/2}(z), E = (Z[k] + conj Z[N/2-k]) / 2 and
-// O = -i (Z[k] - conj Z[N/2-k]) / 2,
-//   X[k] = E + w_N^{-k} O,   X[N/2 - k] = conj(E - w_N^{-k} O),
-// and X[N - k] = conj X[k] (real input). Thread k in [0, N/4] writes bins
-// k, N/2 - k, N/2 + k and N - k, so all N bins are written once.
-__global__ void k_r2c_split(const FwdJob* __restrict__ jobs, FwdJob one, int log2N, const float2* __restrict__ tw) {
-    const FwdJob J = jobs ? jobs[blockIdx.y] : one;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int N = 1 << log2N;
-    const int H = N >> 1;
-    if (k > N / 4) return;
-    const float2* __restrict__ Z = J.tmp;
-    float2* __restrict__ X = J.X;
-    const float2 A = Z[k];
-    const float2 Bz = Z[(H - k) & (H - 1)];
-    const float2 E = make_float2(0.5f * (A.x + Bz.x), 0.5f * (A.y - Bz.y));
-    const float2 O = make_float2(0.5f * (A.y + Bz.y), -0.5f * (A.x - Bz.x));
-    const float2 wo = cmul(fft_tw<-1>(tw, log2N, (unsigned)k), O);
-    const float2 xk = make_float2(E.x + wo.x, E.y + wo.y);
-    const float2 yk = make_float2(E.x - wo.x, wo.y - E.y);
-    X[k] = xk;
-    if (J.log2R && k < H) J.Xp[perm_bin(k, J.log2R)] = xk;
-    if (k == 0) {
-        X[H] = yk;
-        return;
-    }
-    X[N - k] = make_float2(xk.x, -xk.y);
-    if (2 * k < H) {
-        X[H - k] = yk;
-        if (J.log2R) J.Xp[perm_bin(H - k, J.log2R)] = yk;
-        X[H + k] = make_float2(yk.x, -yk.y);
-    }
-}
-
 }  // namespace dev
 
 cudaError_t fft_configure() {
-    cudaError_t e = cudaFuncSetAttribute(dev::k_fft_cols<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(dev::k_fft_cols<-1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          dev::kFftSmemBytes);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(dev::k_adjoint_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kFftSmemBytes);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(dev::k_fft_cols<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kFftSmemBytes);
+    e = cudaFuncSetAttribute(dev::k_fft_cols<-1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kFftSmemBytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(dev::k_fft_cols<+1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kFftSmemBytes);
 }
 
 // FFTs of njobs signals of length N = 2^log2N (jobs in device memory, or
 // `one` for a single signal). SIGN -1: forward, real inputs (real) as r2c
-// when N >= 4, result in each job's X (all N bins); SIGN +1: unnormalised
-// inverse of complex inputs. tw: the two-level table of N.
+// when N >= 4, result in each job's X (complex inputs: all N bins, real ones: the
+// bins up to N / 2); SIGN +1: unnormalised inverse of complex inputs. zero: n_zero words
+// that the first kernel clears. tw: the two-level table of N.
 template <int SIGN>
 static cudaError_t fft_signals(const FwdJob* jobs, const FwdJob& one, int njobs, int log2N, const float2* tw,
-                               bool real, cudaStream_t st, int* n_kernels) {
+                               bool real, cudaStream_t st, int* n_kernels, unsigned* zero = nullptr, int n_zero = 0) {
     *n_kernels = 0;
     if (njobs <= 0) return cudaSuccess;
     if (log2N < 1) return cudaErrorInvalidValue;
@@ -356,42 +382,39 @@ static cudaError_t fft_signals(const FwdJob* jobs, const FwdJob& one, int njobs,
         const int log2cols = log2C - log2L;
         // B = 2^log2B columns per CTA: at most 4096 / L, at most 8, and no more
         // than leaves about two CTAs per SM when there are enough columns
+        const bool split = r2c && dst == 1;
         int log2B = std::min(3, std::min(dev::kFftMaxLog2Tile - log2L, log2cols));
         while (log2B > 2 && ((long long)njobs << (log2cols - log2B)) < dev::kFftTargetCtas) log2B--;
+        // (the split takes columns in pairs: log2B >= 1 unless there is one column)
         const int tile = 1 << (log2L + log2B);
         dim3 grid(1u << (log2cols - log2B), (unsigned)njobs);
-        dev::k_fft_cols<SIGN><<<grid, dev::kFftThreads, (size_t)tile * 16, st>>>(jobs, one, src, dst, log2C, log2L,
-                                                                                   log2B, mode, r2c, tw, log2N);
+        unsigned* z = *n_kernels == 0 ? zero : nullptr;
+        if constexpr (SIGN < 0) {
+            if (split)
+                dev::k_fft_cols<SIGN, true><<<grid, dev::kFftThreads, (size_t)tile * 16, st>>>(
+                    jobs, one, src, dst, log2C, log2L, log2B, mode, r2c, tw, log2N, z, n_zero);
+        }
+        if (!split)
+            dev::k_fft_cols<SIGN, false><<<grid, dev::kFftThreads, (size_t)tile * 16, st>>>(
+                jobs, one, src, dst, log2C, log2L, log2B, mode, r2c, tw, log2N, z, n_zero);
         (*n_kernels)++;
         return cudaGetLastError();
     };
     cudaError_t e;
-    // the last pass writes X, or tmp when the split follows; pass A of r2c
-    // writes into X (free until the split)
-    const int last = r2c ? 2 : 1;
-    if (log2C <= dev::kFftMaxLog2Tile) {
-        e = pass(0, last, log2C, 1);
-    } else {
-        const int log2C2 = log2C / 2;  // pass A length (C2 <= C1)
-        e = pass(0, r2c ? 1 : 2, log2C2, 0);
-        if (e == cudaSuccess) e = pass(r2c ? 1 : 2, last, log2C - log2C2, 1);
-    }
-    if (e != cudaSuccess) return e;
-    if (r2c) {
-        const int threads = (1 << log2N) / 4 + 1;
-        dev::k_r2c_split<<<dim3((threads + 255) / 256, (unsigned)njobs), 256, 0, st>>>(jobs, one, log2N, tw);
-        (*n_kernels)++;
-        e = cudaGetLastError();
-    }
-    return e;
+    if (log2C <= dev::kFftMaxLog2Tile) return pass(0, 1, log2C, 1);
+    const int log2C2 = log2C / 2;  // pass A length (C2 <= C1)
+    e = pass(0, 2, log2C2, 0);
+    return e == cudaSuccess ? pass(2, 1, log2C - log2C2, 1) : e;
 }
 
 cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log2N, const float2* tw,
-                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R) {
+                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R,
+                           unsigned* zero, int n_zero) {
     *n_kernels = 0;
     if (log2N == 0) {
         // N == 1: the DFT is the identity (one sample or none).
         cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float2), st);
+        if (e == cudaSuccess && n_zero > 0) e = cudaMemsetAsync(zero, 0, (size_t)n_zero * sizeof(unsigned), st);
         if (e != cudaSuccess) return e;
         if (n >= 1) {
             if (in_r)
@@ -411,13 +434,13 @@ cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log
     one.tmp = tmp;
     one.Xp = Xp;
     one.gain = nullptr;
-    return fft_signals<-1>(nullptr, one, 1, log2N, tw, in_r != nullptr, st, n_kernels);
+    return fft_signals<-1>(nullptr, one, 1, log2N, tw, in_r != nullptr, st, n_kernels, zero, n_zero);
 }
 
 cudaError_t launch_forward_batched(const FwdJob* jobs, int njobs, int log2N, const float2* tw, cudaStream_t st,
-                                   int* n_kernels, bool real) {
+                                   int* n_kernels, bool real, unsigned* zero, int n_zero) {
     FwdJob none{};
-    return fft_signals<-1>(jobs, none, njobs, log2N, tw, real, st, n_kernels);
+    return fft_signals<-1>(jobs, none, njobs, log2N, tw, real, st, n_kernels, zero, n_zero);
 }
 
 // The adjoint's row FFTs for N > 16384: pass A of `njobs` = batch x rows gradient
@@ -429,8 +452,9 @@ cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int 
     const int log2C2 = log2N / 2, log2C1 = log2N - log2C2;
     FwdJob none{};
     int log2B = std::min(3, dev::kFftMaxLog2Tile - log2C2);
-    dev::k_fft_cols<-1><<<dim3(1u << (log2C1 - log2B), (unsigned)(batch * rows)), dev::kFftThreads,
-                          (size_t)16 << (log2C2 + log2B), st>>>(jobs, none, 0, 2, log2N, log2C2, log2B, 0, 0, tw, log2N);
+    dev::k_fft_cols<-1, false><<<dim3(1u << (log2C1 - log2B), (unsigned)(batch * rows)), dev::kFftThreads,
+                          (size_t)16 << (log2C2 + log2B), st>>>(jobs, none, 0, 2, log2N, log2C2, log2B, 0, 0, tw, log2N,
+                                                                          nullptr, 0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     log2B = std::min(3, dev::kFftMaxLog2Tile - log2C1);

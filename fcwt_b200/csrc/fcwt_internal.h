@@ -135,7 +135,7 @@ struct EngineParams {
     int n_rows;
     void* outs[kMaxOuts];      // output buffers (passed by value with the launch)
     int out_type;
-    int* err;                  // device error word (0 = ok)
+    int* err;                  // error word (0 = ok)
     int tma_store;             // phase-2 outputs via the tensor map (buffer 0, complex64, even n)
 };
 

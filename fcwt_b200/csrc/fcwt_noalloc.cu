@@ -42,7 +42,8 @@ namespace fcwt {
 cudaError_t launch_mother(float fb, int N, float norm, float* out, cudaStream_t st);
 cudaError_t launch_twiddle(int log2N, float2* tw, cudaStream_t st);
 cudaError_t launch_forward(const float* in_r, const float2* in_c, int n, int log2N, const float2* tw,
-                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R);
+                           float2* out, float2* tmp, cudaStream_t st, int* n_kernels, float2* Xp, int log2R,
+                           unsigned* zero = nullptr, int n_zero = 0);
 cudaError_t engine_configure();
 cudaError_t engine_blocks_per_sm(int* out);
 cudaError_t launch_engine(const EngineParams& p, int grid, cudaStream_t st);

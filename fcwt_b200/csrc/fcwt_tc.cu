@@ -180,7 +180,7 @@ __device__ __forceinline__ void mbar_wait_slow(uint32_t mbar, uint32_t parity, i
     const unsigned long long t0 = global_ns();
     while (!mbar_try(mbar, parity)) {
         if (global_ns() - t0 > kWaitLimitNs) {
-            atomicOr(err, kErrWaitTimeout);
+            *(volatile int*)err = *(volatile int*)err | kErrWaitTimeout;  // (may be host memory: no atomics)
             return;
         }
     }

@@ -322,3 +322,23 @@ def test_whole_row_sizes(fcwt, oracle, n, dec, cplx):
     ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)[:, ::dec]
     for r in range(fn):
         assert np.linalg.norm(got[r] - ref[r]) <= 3.5e-6 * np.linalg.norm(ref[r]) + 1e-30, r
+
+
+@pytest.mark.parametrize("n", [4, 5, 8192, 8193, 32767, 65537, 300001])
+def test_real_spectrum_up_to_nyquist(fcwt, oracle, n):
+    """Real inputs whose rows together use nearly all bins up to N / 2, at lengths of
+    one and of two forward passes. Bound: 2 x 19 butterfly levels of 2^-24, 10 twiddles
+    of 2^-22 and split-FP16 products of 2^-21: 5.1e-6 if all were to add up."""
+    import torch
+
+    fn = 6
+    sc = fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LINFREQS, 1000, 20, 499, fn)
+    x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    plan = fcwt.Plan(n, sc, fb=2.0)
+    out = torch.full(plan.out_shape, float("nan"), dtype=torch.complex64, device="cuda")
+    plan.execute(torch.from_numpy(x).cuda(), out)
+    got = out.cpu().numpy()
+    plan.close()
+    ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)
+    for r in range(fn):
+        assert np.linalg.norm(got[r] - ref[r]) <= 5.1e-6 * np.linalg.norm(ref[r]) + 1e-30, r
