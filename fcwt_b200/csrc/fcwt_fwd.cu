@@ -173,12 +173,14 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
     const int tot = L << log2B;
     const int log2H = SPLIT && log2S > 0 ? log2B - 1 : log2B;  // columns of the CTA's own, without the partners
     const int c0 = blockIdx.x << log2H;
+    grid_dep_launch();
     if (zero && blockIdx.x == 0 && blockIdx.y == 0)
         for (int t = threadIdx.x; t < n_zero; t += kFftThreads) zero[t] = 0;
     float2* a = fft_sm;
     float2* b = fft_sm + tot;
     const float2* src = J.tmp;
     stage_tw_fill<SIGN>(tl, tw, log2T, log2L);
+    grid_dep_wait();  // (pass B: pass A's results)
     for (int t = threadIdx.x; t < tot; t += kFftThreads) {
         int i, cc;
         if (mode == 0) {
@@ -389,15 +391,17 @@ static cudaError_t fft_signals(const FwdJob* jobs, const FwdJob& one, int njobs,
         const int tile = 1 << (log2L + log2B);
         dim3 grid(1u << (log2cols - log2B), (unsigned)njobs);
         unsigned* z = *n_kernels == 0 ? zero : nullptr;
+        auto kernel = dev::k_fft_cols<SIGN, false>;
         if constexpr (SIGN < 0) {
-            if (split)
-                dev::k_fft_cols<SIGN, true><<<grid, dev::kFftThreads, (size_t)tile * 16, st>>>(
-                    jobs, one, src, dst, log2C, log2L, log2B, mode, r2c, tw, log2N, z, n_zero);
+            if (split) kernel = dev::k_fft_cols<SIGN, true>;
         }
-        if (!split)
-            dev::k_fft_cols<SIGN, false><<<grid, dev::kFftThreads, (size_t)tile * 16, st>>>(
-                jobs, one, src, dst, log2C, log2L, log2B, mode, r2c, tw, log2N, z, n_zero);
         (*n_kernels)++;
+        if (src == 2)
+            return launch_dependent(kernel, grid, dim3(dev::kFftThreads), (size_t)tile * 16, st, jobs, one, src, dst, log2C,
+                                    log2L, log2B, mode, r2c, tw, log2N, z, n_zero);
+        // (the first pass starts after all that is in the stream: later kernels count on it)
+        kernel<<<grid, dev::kFftThreads, (size_t)tile * 16, st>>>(jobs, one, src, dst, log2C, log2L, log2B, mode, r2c, tw,
+                                                                  log2N, z, n_zero);
         return cudaGetLastError();
     };
     cudaError_t e;

@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(512) k_rows_small(const SigDesc* __restrict__ 
     const int log2T = min(log2L, kSmallTabLog2);
     for (int j = threadIdx.x; j < 1 << log2T; j += blockDim.x) ts[small_pos(j)] = tw_lookup(S.tw, log2N, (unsigned)j << (log2N - log2T));
     float2* a = small_sm;
+    grid_dep_wait();  // (what follows reads the spectrum)
     const float nm1 = (float)N - 1.0f;
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
         float2 z = make_float2(0.0f, 0.0f);
@@ -152,8 +153,8 @@ static cudaError_t small_launch(const SigDesc* sigs, const RowDesc* rows, const 
                                 const OutPtrs& outs, int log2L, cudaStream_t st) {
     // a stage's 16 values per thread, or 8 while that keeps the CTA small (shorter chains)
     const int threads = std::max(64, std::max(std::min(128, 1 << std::max(0, log2L - 3)), 1 << std::max(0, log2L - 4)));
-    dev::k_rows_small<OT><<<(unsigned)n_list, (unsigned)threads, small_smem(log2L), st>>>(sigs, rows, list, pool, outs);
-    return cudaGetLastError();
+    return launch_dependent(dev::k_rows_small<OT>, dim3((unsigned)n_list), dim3((unsigned)threads), small_smem(log2L),
+                            st, sigs, rows, list, pool, outs);
 }
 
 // Rows of N <= 8192 in `list` (null: rows 0 .. n_list - 1); log2L: the largest

@@ -454,7 +454,7 @@ __device__ __forceinline__ float tc_prepass(const TcParams& P, const RowDesc& Rw
     const int k2 = (n >> kLogR) + 16 * (n & (R - 1));
     const unsigned len = (unsigned)(Rw.hi - Rw.lo);
     const float* __restrict__ wrow = P.wts + Rw.woff + n;
-    const float2* __restrict__ xrow = S.Xp + Rw.L + n;
+    const float2* xrow = S.Xp + Rw.L + n;  // (plain loads: read-only ones may be moved above grid_dep_wait)
     const int u0 = Rw.L + k2 - Rw.lo;  // a bin is in [lo, hi) when (unsigned)(u0 + its offset) < len
     struct Load {
         float2 v[16];
@@ -472,7 +472,7 @@ __device__ __forceinline__ float tc_prepass(const TcParams& P, const RowDesc& Rw
             d.m[j] = 0.0f;
             if ((unsigned)(u + o) < len) {
                 d.m[j] = __ldg(wp + o);
-                d.v[j] = __ldg(xp + o);
+                d.v[j] = xp[o];
             }
         }
     };
@@ -692,10 +692,10 @@ struct TcShared {
     UnitSlot u[kTcSlots];
 };
 
-// Claims the CTA's next unit from the queue and pulls its weights and spectrum
-// window into L2.
-__device__ __forceinline__ void tc_claim_next(const TcParams& P, UnitSlot& U) {
-    const int i = (int)atomicAdd(P.counter, 1u);
+// Claims the CTA's next unit and pulls its weights and spectrum window into L2: first
+// the unit of its block index, then the queue's.
+__device__ __forceinline__ void tc_claim_next(const TcParams& P, UnitSlot& U, bool first) {
+    const int i = first ? (int)blockIdx.x : (int)(gridDim.x + atomicAdd(P.counter, 1u));
     U.idx = i;
     if (i < P.n_list) {
         const int e = P.row_list[i];
@@ -776,7 +776,6 @@ __device__ __forceinline__ void produce(const TcParams& P, TcShared& sh, unsigne
             break;
         }
         const ColGeo G = col_geo(U.R, U.S);
-        if (ptid == kTcProdThreads - 32) tc_claim_next(P, sh.u[(k + 1) & (kTcSlots - 1)]);
         int sb, se;
         tc_unit_tiles(U.unit, G.NT, &sb, &se);
         // where Z goes, once nothing reads it any more
@@ -793,6 +792,20 @@ __device__ __forceinline__ void produce(const TcParams& P, TcShared& sh, unsigne
                 for (int j = ptid; j < M; j += kTcProdThreads) twhi_s[j] = U.S.tw[kP2 + j];
             cur_log2N = U.S.log2N;
         }
+        bool a_pending = false;
+        if (k == 0) {
+            // All that does not read the forward transform's results runs under its last
+            // kernel: the tables above, the first operand table and the claim of the unit.
+            acur = P.atab + U.R.aoff + (long long)tile_b(G, sb) * kTcTabBytes;
+            if (ptid == 0) {
+                // (the pass-2 twiddles behind the columns' are the same in every table: once)
+                load_a(a0, acur, kTcColBytes + kTcS2Bytes, smem_u32(&sh.abar));
+                load_col(a0, acur, kTcColBytes + kTcS2Bytes, smem_u32(&sh.abar));
+            }
+            a_pending = true;
+            grid_dep_wait();
+        }
+        if (ptid == kTcProdThreads - 32) tc_claim_next(P, sh.u[(k + 1) & (kTcSlots - 1)], false);
         unsigned char* zb = sm + zoff;
         const float inv = U.R.folds > 1 ? tc_prepass<R, 64, true>(P, U.R, U.S, zb, sh.red)
                           : G.KC == 64  ? tc_prepass<R, 64, false>(P, U.R, U.S, zb, sh.red)
@@ -806,17 +819,19 @@ __device__ __forceinline__ void produce(const TcParams& P, TcShared& sh, unsigne
                 prod_bar();
             }
             if (atab != acur) {
-                if (t > 0) mma_done(t - 1);
+                mma_done(t - 1);
                 if (ptid == 0) {
-                    // (the pass-2 twiddles behind the columns' are the same in every table: once)
-                    const int col = kTcColBytes + (acur ? 0 : kTcS2Bytes);
-                    load_a(a0, atab, col, smem_u32(&sh.abar));
+                    load_a(a0, atab, kTcColBytes, smem_u32(&sh.abar));
                     free_all();
-                    load_col(a0, atab, col, smem_u32(&sh.abar));
+                    load_col(a0, atab, kTcColBytes, smem_u32(&sh.abar));
                 }
+                acur = atab;
+                a_pending = true;
+            }
+            if (a_pending) {
                 if (issuer) mbar_wait(smem_u32(&sh.abar), aphase, P.err);
                 aphase ^= 1u;
-                acur = atab;
+                a_pending = false;
             }
             if (s == sb && ptid == 0) mbar_arrive(smem_u32(&sh.meta[k & (kTcSlots - 1)]));
             const int buf = t % NB;
@@ -1041,7 +1056,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_row_tc(const __grid_constant_
                      "r"(kTcTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (tid == kTcColThreads) tc_claim_next(P, sh.u[0]);
+    if (tid == kTcColThreads) tc_claim_next(P, sh.u[0], true);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1118,22 +1133,17 @@ cudaError_t tc_configure() {
 }
 
 template <int R>
-void launch_tc_r(const TcParams& p, int out_type, int grid, cudaStream_t st) {
-    switch (out_type) {
-        case OUT_BF16: dev::k_row_tc<OUT_BF16, R><<<grid, dev::kTcThreads, dev::kTcSmemBytes, st>>>(p); break;
-        case OUT_F16: dev::k_row_tc<OUT_F16, R><<<grid, dev::kTcThreads, dev::kTcSmemBytes, st>>>(p); break;
-        case OUT_POWER: dev::k_row_tc<OUT_POWER, R><<<grid, dev::kTcThreads, dev::kTcSmemBytes, st>>>(p); break;
-        case OUT_DB: dev::k_row_tc<OUT_DB, R><<<grid, dev::kTcThreads, dev::kTcSmemBytes, st>>>(p); break;
-        default: dev::k_row_tc<OUT_C64, R><<<grid, dev::kTcThreads, dev::kTcSmemBytes, st>>>(p); break;
-    }
+cudaError_t launch_tc_r(const TcParams& p, int out_type, int grid, cudaStream_t st) {
+    auto kernel = out_type == OUT_BF16    ? dev::k_row_tc<OUT_BF16, R>
+                  : out_type == OUT_F16   ? dev::k_row_tc<OUT_F16, R>
+                  : out_type == OUT_POWER ? dev::k_row_tc<OUT_POWER, R>
+                  : out_type == OUT_DB    ? dev::k_row_tc<OUT_DB, R>
+                                          : dev::k_row_tc<OUT_C64, R>;
+    return launch_dependent(kernel, dim3((unsigned)grid), dim3(dev::kTcThreads), (size_t)dev::kTcSmemBytes, st, p);
 }
 
 cudaError_t launch_tc(const TcParams& p, int log2R, int out_type, int grid, cudaStream_t st) {
-    if (log2R == 4)
-        launch_tc_r<16>(p, out_type, grid, st);
-    else
-        launch_tc_r<8>(p, out_type, grid, st);
-    return cudaGetLastError();
+    return log2R == 4 ? launch_tc_r<16>(p, out_type, grid, st) : launch_tc_r<8>(p, out_type, grid, st);
 }
 
 }  // namespace fcwt
