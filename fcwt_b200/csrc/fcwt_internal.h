@@ -90,8 +90,8 @@ constexpr int kWideChunk = kThreads / 32;
 struct Item {
     int type;
     int row;
-    int part;   // chunk / column-group index
-    int pad;
+    int part;   // first chunk (of kChunk or kWideChunk k2) or column group
+    int count;  // how many of them
 };
 
 enum OutType : int { OUT_C64 = 0, OUT_BF16 = 1, OUT_F16 = 2, OUT_POWER = 3, OUT_DB = 4 };
@@ -176,7 +176,6 @@ struct TcParams {
 
 // Error bits written by device code into EngineParams::err.
 constexpr int kErrWaitTimeout = 1;
-constexpr int kErrBadItem = 2;
 
 // ---------------------------------------------------------------- host side
 // Implemented in fcwt_host.cpp (no CUDA dependency).

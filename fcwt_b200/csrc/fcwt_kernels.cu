@@ -70,7 +70,8 @@ constexpr int kSmemFloat2 = kRegion0 + kZs + kP2 + kP2 + kTwhiSmem;
 constexpr size_t kSmemAlign = 1024;  // the 64B-swizzled staging tile wants 1 KB alignment
 constexpr size_t kEngineSmemBytes = (size_t)kSmemFloat2 * sizeof(float2) + kSmemAlign;
 static_assert(4 * kBoxBytes <= kRegion0 * 8, "staging boxes fit in region0");
-constexpr int kFetchBatch = 2;  // work items claimed per queue access
+// Threads of different warps; thread 0 claims items and issues the bulk stores.
+constexpr int kWaiter = 64, kSignaller = 32;
 static_assert(kRegion0 >= (kThreads / 32) * 32 * 33, "per-warp transposes live in region0");
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -378,11 +379,14 @@ __device__ void phase1_wide_dispatch(int K, const SigDesc& S, const RowDesc& R, 
 
 // Warp-level 1024-point DFT (sign +): on entry lane l holds x[m] = G[l + 32 m];
 // on exit lane l holds x[h] = Y[l + 32 h]. tbuf: 32*33 float2 of this warp.
+// before_smem runs when the first half is done in registers.
+template <typename F>
 __device__ __forceinline__ void dft1024_warp(float2 (&x)[32], int lane, float2* __restrict__ tbuf,
-                                             const float2* __restrict__ t2) {
+                                             const float2* __restrict__ t2, F before_smem) {
     fft_reg<32, +1>(x);
 #pragma unroll
     for (int a = 1; a < 32; a++) x[a] = cmul(x[a], t2[a * 32 + lane]);
+    before_smem();
 #pragma unroll
     for (int a = 0; a < 32; a++) tbuf[a * 33 + lane] = x[a];
     __syncwarp();
@@ -413,7 +417,14 @@ __device__ __forceinline__ void phase2_item(const float2* __restrict__ G, int c0
     float2 x[32];
 #pragma unroll
     for (int m = 0; m < 32; m++) x[m] = __ldcg(col + 32 * m);
-    dft1024_warp(x, lane, region0 + warp * (32 * 33), t2);
+    // region0 may still be read by the bulk stores of the previous columns: their end is
+    // waited for only here, under the loads and the first half of the DFT
+    dft1024_warp(x, lane, region0 + warp * (32 * 33), t2, [&]() {
+        if (tma) {
+            if (tid == 0) bulk_wait_read_all();
+            __syncthreads();
+        }
+    });
     __syncthreads();
     const long long row0 = out_off + c0;
     if (tma) {
@@ -472,12 +483,12 @@ __global__ void __launch_bounds__(kThreads, 2)
     float2* twlo = zs + kZs;
     float2* t2 = twlo + kP2;
     float2* twhi_s = t2 + kP2;
-    __shared__ int s_item;
+    __shared__ int s_item[2];
     __shared__ int s_log2N;
     __shared__ int s_ok;
-    __shared__ RowDesc s_rows[kFetchBatch];
-    __shared__ SigDesc s_sigs[kFetchBatch];
-    __shared__ Item s_its[kFetchBatch];
+    __shared__ RowDesc s_rows[2];
+    __shared__ SigDesc s_sigs[2];
+    __shared__ Item s_its[2];
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
@@ -495,40 +506,33 @@ __global__ void __launch_bounds__(kThreads, 2)
     unsigned* a_done = P.counters + 1;
     unsigned* b_done = P.counters + 1 + P.n_rows;
 
-    // Items are claimed kFetchBatch at a time (one atomic and one round of
-    // descriptor loads per batch) and processed in claim order.
-    for (;;) {
+    // Thread 0 claims the items, each while the previous one runs (the descriptors of two
+    // alternate in shared memory), and a barrier makes the claim visible.
+    int next = 0;
+    if (tid == 0) next = (int)atomicAdd(P.counters, 1u);
+    for (int slot = 0;; slot ^= 1) {
         if (tid == 0) {
-            const int i = (int)atomicAdd(P.counters, (unsigned)kFetchBatch);
-            s_item = i;
-#pragma unroll
-            for (int b = 0; b < kFetchBatch; b++)
-                if (i + b < P.n_items) s_its[b] = P.items[i + b];
-#pragma unroll
-            for (int b = 0; b < kFetchBatch; b++)
-                if (i + b < P.n_items) s_rows[b] = P.rows[s_its[b].row];
-#pragma unroll
-            for (int b = 0; b < kFetchBatch; b++)
-                if (i + b < P.n_items) s_sigs[b] = P.sigs[s_rows[b].sig];
+            s_item[slot] = next;
+            if (next < P.n_items) {
+                s_its[slot] = P.items[next];
+                s_rows[slot] = P.rows[s_its[slot].row];
+                s_sigs[slot] = P.sigs[s_rows[slot].sig];
+                next = (int)atomicAdd(P.counters, 1u);  // (used in the next round)
+            }
         }
         __syncthreads();
-        if (s_item >= P.n_items) break;
-      for (int bi = 0; bi < kFetchBatch && s_item + bi < P.n_items; bi++) {
-        const Item& item = s_its[bi];
-        const RowDesc& R = s_rows[bi];
-        const SigDesc& S = s_sigs[bi];
+        if (s_item[slot] >= P.n_items) break;
+        const Item& item = s_its[slot];
+        const RowDesc& R = s_rows[slot];
+        const SigDesc& S = s_sigs[slot];
         const int log2N = S.log2N;
         const int N = 1 << log2N;
-        const int n = S.n;
         void* outb = P.outs[R.out_buf];
         const int Mcols = N >> kLog2P2;
         const TwM twhi = Mcols <= kTwhiSmem ? TwM{twhi_s, nullptr} : TwM{twhi_s, twhi_s + 32};
 
         // region0 may still be read by the bulk stores of the previous phase-2 item
-        if (P.tma_store && (item.type == ITEM_PHASE2 || item.type == ITEM_PHASE1W)) {
-            if (tid == 0) bulk_wait_read_all();
-            __syncthreads();
-        }
+        if (P.tma_store && item.type == ITEM_PHASE1W && tid == 0) bulk_wait_read_all();
         // twiddle tables of this N into SMEM
         if (s_log2N != log2N) {
             for (int j = tid; j < kP2; j += kThreads) twlo[j] = S.tw[j];
@@ -538,57 +542,36 @@ __global__ void __launch_bounds__(kThreads, 2)
                 for (int j = tid; j < 32; j += kThreads) twhi_s[j] = S.tw[kP2 + j];
                 for (int j = tid; j < Mcols / 32; j += kThreads) twhi_s[32 + j] = S.tw[kP2 + 32 * j];
             }
-            __syncthreads();
-            if (tid == 0) s_log2N = log2N;
         }
-
-        if (item.type == ITEM_PHASE1) {
-            if (tid == 0) {
-                s_ok = 1;
-                if (R.wait_row >= 0)
-                    s_ok = wait_counter(b_done + R.wait_row, (unsigned)P.rows[R.wait_row].n_b, P.err) ? 1 : 0;
-            }
-            __syncthreads();
-            if (s_ok) {
-                float2* G = P.scratch + (size_t)R.slot * (size_t)P.slot_elems;
-                phase1_chunk_dispatch(R.K, S, R, P.stale_pool, item.part * kChunk, zs, twlo, twhi, G);
-                if (tid == 0) {
-                    __threadfence();
-                    red_release_add(a_done + item.row, 1u);
-                }
-            }
-        } else if (item.type == ITEM_PHASE1W) {
-            if (tid == 0) {
-                s_ok = 1;
-                if (R.wait_row >= 0)
-                    s_ok = wait_counter(b_done + R.wait_row, (unsigned)P.rows[R.wait_row].n_b, P.err) ? 1 : 0;
-            }
-            __syncthreads();
-            if (s_ok) {
-                float2* G = P.scratch + (size_t)R.slot * (size_t)P.slot_elems;
-                phase1_wide_dispatch(R.K, S, R, P.stale_pool, item.part * kWideChunk, twlo, twhi, region0, G);
-                if (tid == 0) {
-                    __threadfence();
-                    red_release_add(a_done + item.row, 1u);
-                }
-            }
-        } else if (item.type == ITEM_PHASE2) {
-            if (tid == 0) s_ok = wait_counter(a_done + item.row, (unsigned)R.n_a, P.err) ? 1 : 0;
-            __syncthreads();
-            if (s_ok) {
-                const float2* G = P.scratch + (size_t)R.slot * (size_t)P.slot_elems;
-                phase2_item<OT>(G, item.part * kGroupCols, (N >> kLog2P2) / R.dec, R.n_out, R.dec, outb, R.out_off,
-                                R.out_row, region0, t2, &omap, P.tma_store != 0 && R.out_buf == 0);
-                if (tid == 0) {
-                    __threadfence();
-                    red_release_add(b_done + item.row, 1u);
-                }
-            }
-        } else {
-            if (tid == 0) atomicOr(P.err, kErrBadItem);
+        // The thread that waits for other rows, the one that signals the end (after the
+        // block's last barrier) and the one that claims the next item are of three warps, so
+        // that their latencies overlap.
+        const bool phase1 = item.type == ITEM_PHASE1 || item.type == ITEM_PHASE1W;
+        if (tid == kWaiter) {
+            s_ok = 1;
+            if (phase1 && R.wait_row >= 0)
+                s_ok = wait_counter(b_done + R.wait_row, (unsigned)P.rows[R.wait_row].n_b, P.err) ? 1 : 0;
+            else if (!phase1)
+                s_ok = wait_counter(a_done + item.row, (unsigned)R.n_a, P.err) ? 1 : 0;
         }
         __syncthreads();
-      }
+        if (tid == 0) s_log2N = log2N;
+        if (s_ok) {
+            float2* G = P.scratch + (size_t)R.slot * (size_t)P.slot_elems;
+            for (int c = item.part; c < item.part + item.count; c++) {
+                if (item.type == ITEM_PHASE1)
+                    phase1_chunk_dispatch(R.K, S, R, P.stale_pool, c * kChunk, zs, twlo, twhi, G);
+                else if (item.type == ITEM_PHASE1W)
+                    phase1_wide_dispatch(R.K, S, R, P.stale_pool, c * kWideChunk, twlo, twhi, region0, G);
+                else
+                    phase2_item<OT>(G, c * kGroupCols, (N >> kLog2P2) / R.dec, R.n_out, R.dec, outb, R.out_off, R.out_row,
+                                    region0, t2, &omap, P.tma_store != 0 && R.out_buf == 0);
+            }
+            if (tid == kSignaller) {
+                __threadfence();
+                red_release_add((phase1 ? a_done : b_done) + item.row, 1u);
+            }
+        }
     }
     if (tid == 0 && P.tma_store) bulk_wait_all();
 }

@@ -120,10 +120,10 @@ __global__ void k_na_items(int fn, int n_a, int n_b, int lag, Item* __restrict__
     if (s >= fn + lag) return;
     int base = n_a * min(s, fn) + n_b * max(0, min(s - lag, fn));
     if (s < fn)
-        for (int a = 0; a < n_a; a++) items[base++] = Item{ITEM_PHASE1, s, a, 0};
+        for (int a = 0; a < n_a; a++) items[base++] = Item{ITEM_PHASE1, s, a, 1};
     const int rb = s - lag;
     if (rb >= 0 && rb < fn)
-        for (int b = 0; b < n_b; b++) items[base++] = Item{ITEM_PHASE2, rb, b, 0};
+        for (int b = 0; b < n_b; b++) items[base++] = Item{ITEM_PHASE2, rb, b, 1};
 }
 
 int na_fail(int code, const std::string& msg) {

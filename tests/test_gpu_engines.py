@@ -342,3 +342,24 @@ def test_real_spectrum_up_to_nyquist(fcwt, oracle, n):
     ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)
     for r in range(fn):
         assert np.linalg.norm(got[r] - ref[r]) <= 5.1e-6 * np.linalg.norm(ref[r]) + 1e-30, r
+
+
+@pytest.mark.parametrize("n,dec", [((1 << 20) - 3, 1), (1 << 20, 4)])
+def test_wide_rows_of_several_chunks_per_item(fcwt, oracle, n, dec):
+    """Enough wide rows that a work item takes several chunks of a row. Bound: 2 x 20
+    butterfly levels of 2^-24 and 10 twiddles of 2^-22: 4.8e-6 if all were to add up."""
+    import torch
+
+    fn, rows = 44, [0, 21, 43]
+    sc = fcwt.Scales(fcwt.Morlet(4.0), fcwt.FCWT_LINFREQS, 200000, 8000, 80000, fn)
+    x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    plan = fcwt.Plan(n, sc, fb=4.0, time_stride=dec)
+    assert plan.stats()["tensor_core_rows"] == 0
+    out = torch.full(plan.out_shape, float("nan"), dtype=torch.complex64, device="cuda")
+    plan.execute(torch.from_numpy(x).cuda(), out)
+    got = out[rows].cpu().numpy()
+    assert not bool(torch.isnan(torch.view_as_real(out)).any())
+    plan.close()
+    ref = oracle.cwt_fp64(x, sc.scales, 4.0, 1, True, rows=rows)[:, ::dec]
+    for r in range(len(rows)):
+        assert rel_l2(got[r], ref[r]) <= 4.8e-6, rows[r]
