@@ -383,10 +383,12 @@ static cudaError_t fft_signals(const FwdJob* jobs, const FwdJob& one, int njobs,
     auto pass = [&](int src, int dst, int log2L, int mode) -> cudaError_t {
         const int log2cols = log2C - log2L;
         // B = 2^log2B columns per CTA: at most 4096 / L, at most 8, and no more
-        // than leaves about two CTAs per SM when there are enough columns
+        // than leaves about two CTAs per SM when there are enough columns (down to two:
+        // one signal of 131072 is bound by latency; with four columns at least, a call of
+        // 99991 x 300 took 183 us, with two 180)
         const bool split = r2c && dst == 1;
         int log2B = std::min(3, std::min(dev::kFftMaxLog2Tile - log2L, log2cols));
-        while (log2B > 2 && ((long long)njobs << (log2cols - log2B)) < dev::kFftTargetCtas) log2B--;
+        while (log2B > 1 && ((long long)njobs << (log2cols - log2B)) < dev::kFftTargetCtas) log2B--;
         // (the split takes columns in pairs: log2B >= 1 unless there is one column)
         const int tile = 1 << (log2L + log2B);
         dim3 grid(1u << (log2cols - log2B), (unsigned)njobs);
