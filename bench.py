@@ -59,7 +59,7 @@ THREADS = os.cpu_count() or 1
 # output type, from one-pass ncu captures of the full-size launch
 # (dram__bytes_read.sum + dram__bytes_write.sum; the capture summaries are
 # kept under profiles/, named for the kernel and the workload)
-TRAFFIC_PER_LAUNCH = {"complex64": 147.96e6 + 2.34565e9, "bf16": 156.01e6 + 1.14550e9}
+TRAFFIC_PER_LAUNCH = {"complex64": 131.76e6 + 2.34043e9, "bf16": 132.16e6 + 1.13992e9}
 
 # --out choices: (constant in fcwt_b200, trailing shape, torch dtype, bytes per point)
 OUT_TYPES = {

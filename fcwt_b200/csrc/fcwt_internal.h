@@ -9,7 +9,8 @@
 // for proc_i <= q the weight the most recent earlier row wrote into the reused
 // O1 buffer (0 if none). idx_i(q) = (int)min(N-1, (float)(scale_i/2) * q).
 //
-// Device decomposition of the inverse transform, per row, with P2 = 1024:
+// Device decomposition of the inverse transform in the CUDA-core engine, per row, with
+// P2 = 1024 (the tensor-core engine: fcwt_tc.cu):
 //   t = c + M*a      (c < M = N/1024 columns, a < 1024)
 //   q = L + k2 + 1024*k1   (L a multiple of 1024, k2 < 1024, k1 < K)
 //   phase 1 (per k2, per v < R = M/K):
