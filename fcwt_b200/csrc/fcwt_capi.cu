@@ -1705,19 +1705,23 @@ int fcwt_plan_execute_graph(fcwt_plan* plan, const void* const* inputs, void* co
         key.push_back(outputs[s]);
     }
     cudaStream_t st = ctx->stream;
+    // The graph holds the addresses of the context's workspaces, which all its plans share and
+    // which move when a larger call needs more: they are brought to this plan's size first
+    // (nothing may be allocated during a capture) and their addresses are part of the key.
+    size_t maxN = 1;
+    for (auto& S : plan->sig) maxN = std::max(maxN, (size_t)S.sp.N);
+    FCWT_CUDA_TRY(ctx->tmp.ensure(maxN * sizeof(float2)));
+    FCWT_CUDA_TRY(ctx->counters.ensure(plan_counters(plan) * sizeof(unsigned)));
+    FCWT_CUDA_TRY(ctx->err.ensure(sizeof(int)));
+    if (plan->two_phase)
+        FCWT_CUDA_TRY(ctx->scratch.ensure((size_t)plan->slots * (size_t)plan->slot_elems * sizeof(float2)));
+    for (const DevBuf* b : {&ctx->tmp, &ctx->counters, &ctx->err}) key.push_back(b->p);
+    key.push_back(plan->two_phase ? ctx->scratch.p : nullptr);
     if (!plan->graph || key != plan->graph_key || out_type != plan->graph_out_type) {
         if (plan->graph) {
             cudaGraphExecDestroy(plan->graph);
             plan->graph = nullptr;
         }
-        // make sure every buffer the enqueue touches exists before capturing
-        size_t maxN = 1;
-        for (auto& S : plan->sig) maxN = std::max(maxN, (size_t)S.sp.N);
-        FCWT_CUDA_TRY(ctx->tmp.ensure(maxN * sizeof(float2)));
-        FCWT_CUDA_TRY(ctx->counters.ensure(plan_counters(plan) * sizeof(unsigned)));
-        FCWT_CUDA_TRY(ctx->err.ensure(sizeof(int)));
-        if (plan->two_phase)
-            FCWT_CUDA_TRY(ctx->scratch.ensure((size_t)plan->slots * (size_t)plan->slot_elems * sizeof(float2)));
         const fcwt::FwdJob* gj = nullptr;
         if (nsig > 1) {
             // the graph reads its jobs from a buffer of its own,

@@ -203,8 +203,9 @@ int fcwt_plan_create_batched(fcwt_context* ctx, int nsig, const int* ns, int is_
  * signal s is fns[s] x ns[s] values). */
 int fcwt_plan_execute_batched(fcwt_plan* plan, const void* const* inputs, void* const* outputs, int out_type);
 /* Same, for device buffers only, replayed from a CUDA graph: the first call
- * (and any call with different pointers or output type) captures the whole
- * sequence on the context's stream; later calls launch the graph. */
+ * (and any call with different pointers or output type, or after a larger call
+ * on the context has moved its workspaces) captures the whole sequence on the
+ * context's stream; later calls launch the graph. */
 int fcwt_plan_execute_graph(fcwt_plan* plan, const void* const* inputs, void* const* outputs, int out_type);
 
 /* ---- differentiable Morlet CWT (FCWT_CONTINUOUS forward)

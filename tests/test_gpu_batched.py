@@ -188,3 +188,52 @@ def test_context_destroyed_before_its_plans(fcwt, oracle):
     rc = lib.fcwt_plan_execute_batched(h, in_arr, out_arr, fcwt.FCWT_OUT_C64)
     assert rc == _lib.FCWT_ERR_INVALID and b"context" in lib.fcwt_last_error()
     assert lib.fcwt_plan_destroy(h) == 0
+
+
+def test_graph_after_the_workspaces_moved(fcwt, oracle, monkeypatch):
+    """A captured graph holds addresses of the context's workspaces; a larger
+    call in between frees and reallocates them. The next execution captures
+    anew (its kernels are counted again) and its results are the same bits."""
+    import torch
+
+    from fcwt_b200 import _lib
+
+    ctx = _lib.Context(0)  # workspaces of its own, so that the larger call does move them
+    monkeypatch.setitem(_lib._contexts, 0, ctx)
+    rng = np.random.default_rng(12)
+    # two signals with wide rows (scratch ring), and one signal alone (the FFT buffer)
+    lengths, fs = [20000, 120000], 1000
+    grids = [oracle.scales(LOGSCALES, fs, 2.0, 480.0, 20) for _ in lengths]
+    xs = [torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda() for n in lengths]
+    plans = [fcwt.BatchPlan(lengths, grids, fb=6.0), fcwt.BatchPlan(lengths[:1], grids[:1], fb=6.0)]
+    assert plans[0].stats()["tensor_core_rows"] < plans[0].stats()["rows"]
+    big_n = 1 << 20
+    big = fcwt.Plan(big_n, oracle.scales(LOGSCALES, fs, 2.0, 480.0, 400), fb=6.0)
+    big_out = torch.empty((400, big_n), dtype=torch.complex64, device="cuda")
+    big_x = torch.randn(big_n, device="cuda")
+    for bp in plans:
+        ins = xs[:len(bp.ns)]
+        want = bp.outputs_like()
+        bp.execute(ins, want)
+        outs = bp.outputs_like()
+        for _ in range(2):
+            bp.execute(ins, outs, graph=True)
+        fcwt.synchronize()
+        ctx.profile_read()
+        bp.execute(ins, outs, graph=True)
+        fcwt.synchronize()
+        assert ctx.profile_read()[2] == 0  # a replay
+        bp.want, bp.outs = want, outs
+    big.execute(big_x, big_out)
+    for bp in plans:
+        fcwt.synchronize()
+        ctx.profile_read()
+        for t in bp.outs:
+            t.zero_()
+        bp.execute(xs[:len(bp.ns)], bp.outs, graph=True)
+        fcwt.synchronize()
+        assert ctx.profile_read()[2] > 0  # captured again
+        for a, b in zip(bp.outs, bp.want):
+            assert torch.equal(a, b)
+        bp.close()
+    big.close()
