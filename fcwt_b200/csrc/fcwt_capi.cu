@@ -40,9 +40,11 @@ cudaError_t launch_adjoint_accum(const float2* Xs, const float2* Gh, float2* H, 
 cudaError_t launch_take_real(const float2* Y, long long Nstride, int n, int batch, float scale, float* gx,
                              cudaStream_t st);
 int adjoint_rows_per_pass();
-cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int rows, const float2* Xs, const void* rowc,
-                                int log2N, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
-                                double* acc_sigma, double* acc_f, cudaStream_t st);
+int adjoint_long_rows_per_cta(int log2N, int batch, int rows);
+cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int rows, int per, const float2* Xs,
+                                const void* rowc, int log2N, const float2* tw, float cb, float amp, float inv_sigma,
+                                float2* H, float2* part, bool first, double* acc_sigma, double* acc_f, cudaStream_t st);
+cudaError_t launch_adjoint_hsum(float2* H, const float2* part, int nparts, int log2N, int batch, cudaStream_t st);
 cudaError_t launch_adjoint_rows(const float2* G, const float* gain, const float2* Xs, const void* rows, int n, int log2N, int fn,
                                 int batch, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
                                 double* acc_sigma, double* acc_f, cudaStream_t st);
@@ -261,7 +263,7 @@ struct fcwt_context {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_used, ev_free;
     long long kernel_launches = 0;
     // workspace of the differentiable transform's backward
-    DevBuf adj_tw, adj_x, adj_g, adj_tmp, adj_h, adj_jobs, adj_rows, adj_acc;
+    DevBuf adj_tw, adj_x, adj_g, adj_tmp, adj_h, adj_part, adj_jobs, adj_rows, adj_acc;
     int adj_tw_log2N = -1;
     void* adj_jobs_host = nullptr;
     size_t adj_jobs_host_bytes = 0;
@@ -1323,8 +1325,8 @@ int fcwt_context_destroy(fcwt_context* ctx) {
         if (u.host) cudaFreeHost(u.host);
         if (u.done) cudaEventDestroy(u.done);
     }
-    for (DevBuf* b : {&ctx->adj_tw, &ctx->adj_x, &ctx->adj_g, &ctx->adj_tmp, &ctx->adj_h, &ctx->adj_jobs,
-                      &ctx->adj_rows, &ctx->adj_acc})
+    for (DevBuf* b : {&ctx->adj_tw, &ctx->adj_x, &ctx->adj_g, &ctx->adj_tmp, &ctx->adj_h, &ctx->adj_part,
+                      &ctx->adj_jobs, &ctx->adj_rows, &ctx->adj_acc})
         b->release();
     if (ctx->adj_jobs_host) cudaFreeHost(ctx->adj_jobs_host);
     for (auto& ev : ctx->ev_used) {
@@ -1851,6 +1853,10 @@ int fcwt_morlet_power_backward(fcwt_context* ctx, const float* x, int n, int bat
     FCWT_CUDA_TRY(ctx->adj_h.ensure(BN * sizeof(float2)));
     FCWT_CUDA_TRY(ctx->adj_g.ensure(BN * (fused || long_rows ? 1 : RP) * sizeof(float2)));
     FCWT_CUDA_TRY(ctx->adj_tmp.ensure(BN * (fused ? 1 : RP) * sizeof(float2)));
+    // long rows: sums of H that the CTAs keep besides H itself (at most 32 MB)
+    const int per = long_rows ? adjoint_long_rows_per_cta(log2N, batch, std::min(RP, fn)) : 1;
+    const int nparts = long_rows ? (std::min(RP, fn) + per - 1) / per - 1 : 0;
+    if (nparts) FCWT_CUDA_TRY(ctx->adj_part.ensure((size_t)nparts * batch * half * sizeof(float2)));
     const size_t njobs_total = (size_t)batch * (2 + (size_t)fn);
     FCWT_CUDA_TRY(ctx->adj_jobs.ensure(njobs_total * sizeof(FwdJob)));
     if (ctx->adj_jobs_host_bytes < njobs_total * sizeof(FwdJob)) {
@@ -1930,11 +1936,11 @@ int fcwt_morlet_power_backward(fcwt_context* ctx, const float* x, int n, int bat
         }
         FCWT_CUDA_TRY(cudaMemcpyAsync(jd + jo, jh + jo, (size_t)batch * nr * sizeof(FwdJob), cudaMemcpyHostToDevice, st));
         if (long_rows) {
-            FCWT_CUDA_TRY(launch_adjoint_long(jd + jo, ctx->adj_tmp.as<float2>(), batch, nr, ctx->adj_x.as<float2>(),
+            FCWT_CUDA_TRY(launch_adjoint_long(jd + jo, ctx->adj_tmp.as<float2>(), batch, nr, per, ctx->adj_x.as<float2>(),
                                               static_cast<const AdjRowH*>(ctx->adj_rows.p) + i0, log2N, tw,
                                               (float)(two_pi * fb), host::mother_norm(), 1.0f / fb,
-                                              ctx->adj_h.as<float2>(), ctx->adj_acc.as<double>(),
-                                              ctx->adj_acc.as<double>() + 1 + i0, st));
+                                              ctx->adj_h.as<float2>(), ctx->adj_part.as<float2>(), c == 0,
+                                              ctx->adj_acc.as<double>(), ctx->adj_acc.as<double>() + 1 + i0, st));
             ctx->kernel_launches += 2;
             jo += (size_t)batch * nr;
             continue;
@@ -1948,6 +1954,8 @@ int fcwt_morlet_power_backward(fcwt_context* ctx, const float* x, int n, int bat
                                            ctx->adj_acc.as<double>(), ctx->adj_acc.as<double>() + 1 + i0, st));
         ctx->kernel_launches += 1;
     }
+    FCWT_CUDA_TRY(launch_adjoint_hsum(ctx->adj_h.as<float2>(), ctx->adj_part.as<float2>(), nparts, log2N, batch, st));
+    ctx->kernel_launches += nparts > 0 ? 1 : 0;
     // dL/dx = Re(scale * IFFTraw(H))[0:n]
     for (int b = 0; b < batch; b++) {
         FwdJob& j = jh[jo + b];

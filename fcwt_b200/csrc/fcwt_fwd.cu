@@ -268,13 +268,17 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
 // (in registers over its rows) and the sigma and frequency partial sums, so the
 // rows' spectra are never written. (Writing them and reading them back took the
 // second pass 43 us and the sums 11 us per 64 rows of N = 65536.)
+// The CTAs of one bin tile, blockIdx.z, keep sums of their own: z = 0 in H, the others
+// in part[z - 1], which the launches of one backward pass carry on (`first`: start at
+// zero) and k_adjoint_hsum adds in the order of z. So the same call gives the same
+// bits; with float atomics into H the order of the additions varied.
 constexpr int kAdjColPos = (1 << kFftMaxLog2Tile) / 2 / kFftThreads;  // bins per thread, at most
 
 __global__ void __launch_bounds__(kFftThreads)
     k_adjoint_cols(const float2* __restrict__ T, const float2* __restrict__ Xs, const float2* __restrict__ rowc,
                    int rows_total, int rows_per_cta, int log2C, int log2L, int log2B, const float2* __restrict__ tw,
-                   float cb, float amp, float inv_sigma, float2* __restrict__ H, double* __restrict__ acc_sigma,
-                   double* __restrict__ acc_f) {
+                   float cb, float amp, float inv_sigma, float2* __restrict__ H, float2* __restrict__ part, int first,
+                   double* __restrict__ acc_sigma, double* __restrict__ acc_f) {
     extern __shared__ float2 fft_sm[];
     __shared__ float2 tl[kStageTw];
     __shared__ float s_red[kFftThreads / 32][2];
@@ -287,6 +291,8 @@ __global__ void __launch_bounds__(kFftThreads)
     const int r0 = blockIdx.z * rows_per_cta;
     const int nr = min(rows_per_cta, rows_total - r0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2* hsum = blockIdx.z == 0 ? H + ((size_t)b << log2C)
+                                   : part + (((size_t)(blockIdx.z - 1) * gridDim.y + b) << (log2C - 1));
     stage_tw_fill<-1>(tl, tw, log2C, log2L);
     float2 h[kAdjColPos], xq[kAdjColPos];
 #pragma unroll
@@ -296,6 +302,7 @@ __global__ void __launch_bounds__(kFftThreads)
         if (t < pos) {
             const int q = c0 + (t & (B - 1)) + ((t >> log2B) << log2S);
             xq[i] = __ldg(Xs + ((size_t)b << log2C) + q);
+            if (!first) h[i] = hsum[q];
         }
     }
     double dsig = 0.0;
@@ -346,12 +353,27 @@ __global__ void __launch_bounds__(kFftThreads)
 #pragma unroll
     for (int i = 0; i < kAdjColPos; i++) {
         const int t = threadIdx.x + i * kFftThreads;
-        if (t < pos) {
-            float* hp = reinterpret_cast<float*>(H + ((size_t)b << log2C) + c0 + (t & (B - 1)) + ((t >> log2B) << log2S));
-            atomicAdd(hp, h[i].x);
-            atomicAdd(hp + 1, h[i].y);
-        }
+        if (t < pos) hsum[c0 + (t & (B - 1)) + ((t >> log2B) << log2S)] = h[i];
     }
+}
+
+// H += part[0] + part[1] + ... in this order, two bins per thread.
+__global__ void k_adjoint_hsum(float2* __restrict__ H, const float2* __restrict__ part, int nparts, int log2N) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 1 << (log2N - 2)) return;
+    const size_t stride = (size_t)gridDim.y << (log2N - 2);
+    const float4* p = reinterpret_cast<const float4*>(part) + ((size_t)blockIdx.y << (log2N - 2)) + i;
+    float4* hp = reinterpret_cast<float4*>(H) + ((size_t)blockIdx.y << (log2N - 1)) + i;
+    float4 h = *hp;
+#pragma unroll 4
+    for (int z = 0; z < nparts; z++) {
+        const float4 v = __ldcg(p + z * stride);
+        h.x += v.x;
+        h.y += v.y;
+        h.z += v.z;
+        h.w += v.w;
+    }
+    *hp = h;
 }
 
 }  // namespace dev
@@ -449,12 +471,23 @@ cudaError_t launch_forward_batched(const FwdJob* jobs, int njobs, int log2N, con
     return fft_signals<-1>(jobs, none, njobs, log2N, tw, real, st, n_kernels, zero, n_zero);
 }
 
+// Rows a CTA of k_adjoint_cols takes when a launch has `rows` of them: enough CTAs for
+// every SM, H read and written once per CTA.
+int adjoint_long_rows_per_cta(int log2N, int batch, int rows) {
+    const int log2C2 = log2N / 2, log2C1 = log2N - log2C2;
+    const int groups = 1 << (log2C2 - std::min(3, dev::kFftMaxLog2Tile - log2C1));
+    int per = 1;
+    while (per < 16 && per < rows && (long long)groups * batch * ((rows + 2 * per - 1) / (2 * per)) >= 8 * 148) per *= 2;
+    return per;
+}
+
 // The adjoint's row FFTs for N > 16384: pass A of `njobs` = batch x rows gradient
 // rows into consecutive tmp buffers (N values each, from `tmp`), then the fused
-// pass B. rowc: (ca, dfdq) of the rows.
-cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int rows, const float2* Xs, const void* rowc,
-                                int log2N, const float2* tw, float cb, float amp, float inv_sigma, float2* H,
-                                double* acc_sigma, double* acc_f, cudaStream_t st) {
+// pass B. rowc: (ca, dfdq) of the rows; part: ceil(rows / per) - 1 sums of batch x N / 2
+// bins (k_adjoint_cols).
+cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int rows, int per, const float2* Xs,
+                                const void* rowc, int log2N, const float2* tw, float cb, float amp, float inv_sigma,
+                                float2* H, float2* part, bool first, double* acc_sigma, double* acc_f, cudaStream_t st) {
     const int log2C2 = log2N / 2, log2C1 = log2N - log2C2;
     FwdJob none{};
     int log2B = std::min(3, dev::kFftMaxLog2Tile - log2C2);
@@ -464,13 +497,16 @@ cudaError_t launch_adjoint_long(const FwdJob* jobs, float2* tmp, int batch, int 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     log2B = std::min(3, dev::kFftMaxLog2Tile - log2C1);
-    const int groups = 1 << (log2C2 - log2B);
-    // rows per CTA: enough CTAs for every SM, H added once per CTA
-    int per = 1;
-    while (per < 16 && per < rows && (long long)groups * batch * ((rows + 2 * per - 1) / (2 * per)) >= 8 * 148) per *= 2;
-    dev::k_adjoint_cols<<<dim3(groups, batch, (rows + per - 1) / per), dev::kFftThreads, (size_t)16 << (log2C1 + log2B),
-                          st>>>(tmp, Xs, static_cast<const float2*>(rowc), rows, per, log2N, log2C1, log2B, tw, cb, amp,
-                                inv_sigma, H, acc_sigma, acc_f);
+    dev::k_adjoint_cols<<<dim3(1u << (log2C2 - log2B), batch, (rows + per - 1) / per), dev::kFftThreads,
+                          (size_t)16 << (log2C1 + log2B), st>>>(tmp, Xs, static_cast<const float2*>(rowc), rows, per, log2N,
+                                                                log2C1, log2B, tw, cb, amp, inv_sigma, H, part,
+                                                                first ? 1 : 0, acc_sigma, acc_f);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_hsum(float2* H, const float2* part, int nparts, int log2N, int batch, cudaStream_t st) {
+    if (nparts <= 0) return cudaSuccess;
+    dev::k_adjoint_hsum<<<dim3((1u << (log2N - 2)) / 256, (unsigned)batch), 256, 0, st>>>(H, part, nparts, log2N);
     return cudaGetLastError();
 }
 

@@ -210,3 +210,22 @@ def test_long_adjoint_edges(n, B, F, power):
         want = torch.autograd.grad(yr, [xr, sr, fr], G.to(torch.complex128))
     for a, b in zip(got, want):
         assert float(torch.linalg.vector_norm(a.double() - b)) <= 2e-5 * float(torch.linalg.vector_norm(b))
+
+
+# one launch of rows, several with a shorter last one, one row per launch, more rows per CTA than one
+@pytest.mark.parametrize("n,B,F", [(17000, 1, 7), (33000, 8, 40), (40000, 8, 21), (300000, 16, 3), (20001, 2, 96)])
+def test_long_adjoint_repeats_exactly(n, B, F):
+    """Two backward passes of one call give the same signal gradient, bit for bit."""
+    import torch
+
+    from fcwt_b200.autograd import morlet_cwt
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((B, n), generator=g, device="cuda").requires_grad_(True)
+    sigma = torch.tensor(2.0, device="cuda", requires_grad=True)
+    freqs = torch.from_numpy(np.geomspace(8.0, 120.0, F)).float().cuda().requires_grad_(True)
+    y = morlet_cwt(x, sigma, freqs, 1000.0)
+    G = torch.randn(y.shape, generator=g, dtype=torch.complex64, device="cuda")
+    first = torch.autograd.grad(y, x, G, retain_graph=True)[0]
+    for _ in range(4):
+        assert torch.equal(torch.autograd.grad(y, x, G, retain_graph=True)[0], first)
