@@ -60,14 +60,19 @@ __device__ __forceinline__ float2 fft_tw(const float2* __restrict__ tw, int log2
 }
 
 // Stage twiddles of a CTA: w_L^{SIGN j} for j < min(L, 1024); for longer L the factors
-// w_L^{SIGN 1024 j} follow.
+// w_L^{SIGN 1024 j} follow. Each is computed (2 j / L is exact), not looked up: the
+// table of N gives most of them as products of two rounded factors, and the stages
+// multiply them once more (smem_stage).
 constexpr int kStageTw = 1024 + (1 << kFftMaxLog2Tile) / 1024;
 template <int SIGN>
-__device__ __forceinline__ void stage_tw_fill(float2* __restrict__ tl, const float2* __restrict__ tw, int log2T,
-                                              int log2L) {
+__device__ __forceinline__ void stage_tw_fill(float2* __restrict__ tl, int log2L) {
     const int n = log2L <= 10 ? 1 << log2L : 1024 + (1 << (log2L - 10));
-    for (int t = threadIdx.x; t < n; t += kFftThreads)
-        tl[t] = fft_tw<SIGN>(tw, log2T, (unsigned)(t < 1024 ? t : (t - 1024) << 10) << (log2T - log2L));
+    const float step = 2.0f / (float)(1 << log2L);
+    for (int t = threadIdx.x; t < n; t += kFftThreads) {
+        float sn, cs;
+        sincospif((float)(t < 1024 ? t : (t - 1024) << 10) * step, &sn, &cs);
+        tl[t] = make_float2(cs, SIGN < 0 ? -sn : sn);
+    }
 }
 __device__ __forceinline__ float2 stage_tw(const float2* __restrict__ tl, unsigned e) {
     return e < 1024u ? tl[e] : cmul(tl[e & 1023u], tl[1024 + (e >> 10)]);
@@ -179,7 +184,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
     float2* a = fft_sm;
     float2* b = fft_sm + tot;
     const float2* src = J.tmp;
-    stage_tw_fill<SIGN>(tl, tw, log2T, log2L);
+    stage_tw_fill<SIGN>(tl, log2L);
     grid_dep_wait();  // (pass B: pass A's results)
     for (int t = threadIdx.x; t < tot; t += kFftThreads) {
         int i, cc;
@@ -237,24 +242,16 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_cols(const FwdJob* __restri
         return;
     }
     float2* dst = dst_sel == 1 ? J.X : J.tmp;
-    // inter-pass twiddle w_C^{SIGN col k}: a thread's column is fixed and its k goes up
-    // by 128 / B, so the twiddle advances by a factor; looked up again every four
-    // (scattered lookups of both tables at each sample took most of the pass: 94 us
-    // for 128 rows of 65536)
-    const int dk = kFftThreads >> log2B;
-    const int my_col = c0 + (threadIdx.x & (B - 1));
-    float2 w = make_float2(1.0f, 0.0f), wstep = w;
-    if (mode == 0) wstep = fft_tw<SIGN>(tw, log2T, (unsigned)(my_col * dk) << (log2T - log2C));
-    int it = 0;
-    for (int t = threadIdx.x; t < tot; t += kFftThreads, it++) {
+    // Inter-pass twiddle w_C^{SIGN col k}, looked up at each sample. (Stepped by a product
+    // with lookups every four samples, the gradient of 8 x 40000 x 64 took 1.10 ms with its
+    // forward instead of 1.14 but was off by 3.9e-7 of its size instead of 3.5e-7; a call of
+    // 99991 x 300 takes 177 us either way.)
+    for (int t = threadIdx.x; t < tot; t += kFftThreads) {
         const int cc = t & (B - 1);
         const int k = t >> log2B;
         const int col = c0 + cc;
         float2 v = res[t];
-        if (mode == 0) {
-            w = (it & 3) ? cmul(w, wstep) : fft_tw<SIGN>(tw, log2T, (unsigned)(col * k) << (log2T - log2C));
-            v = cmul(v, w);
-        }
+        if (mode == 0) v = cmul(v, fft_tw<SIGN>(tw, log2T, (unsigned)(col * k) << (log2T - log2C)));
         const int o = col + (k << log2S);
         dst[o] = v;
         if (dst_sel == 1 && J.log2R && o < (1 << (log2C - 1))) J.Xp[perm_bin(o, J.log2R)] = v;
@@ -293,7 +290,7 @@ __global__ void __launch_bounds__(kFftThreads)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float2* hsum = blockIdx.z == 0 ? H + ((size_t)b << log2C)
                                    : part + (((size_t)(blockIdx.z - 1) * gridDim.y + b) << (log2C - 1));
-    stage_tw_fill<-1>(tl, tw, log2C, log2L);
+    stage_tw_fill<-1>(tl, log2L);
     float2 h[kAdjColPos], xq[kAdjColPos];
 #pragma unroll
     for (int i = 0; i < kAdjColPos; i++) {

@@ -229,3 +229,29 @@ def test_long_adjoint_repeats_exactly(n, B, F):
     first = torch.autograd.grad(y, x, G, retain_graph=True)[0]
     for _ in range(4):
         assert torch.equal(torch.autograd.grad(y, x, G, retain_graph=True)[0], first)
+
+
+@pytest.mark.parametrize("n,B,F,fmin,fmax", [(20001, 2, 24, 3.0, 120.0), (40000, 8, 64, 2.0, 200.0)])
+def test_long_adjoint_accuracy(n, B, F, fmin, fmax):
+    """The signal gradient of white noise against float64. The bound of 3.75e-7 lies
+    between FFT passes whose inter-pass factors are products of two rounded ones
+    (3.5e-7 to 3.6e-7 of the gradient's size at these lengths) and passes that step
+    them by up to three more products (3.9e-7 to 4.0e-7)."""
+    import torch
+
+    from fcwt_b200.autograd import morlet_cwt
+
+    rng = np.random.default_rng(n)
+    fs = 1000.0
+    x = torch.from_numpy(rng.standard_normal((B, n))).float().cuda().requires_grad_(True)
+    f0 = np.geomspace(fmin, fmax, F).astype(np.float32)
+    sigma = torch.tensor(2.0, device="cuda", requires_grad=True)
+    freqs = torch.from_numpy(f0).cuda().requires_grad_(True)
+    y = morlet_cwt(x, sigma, freqs, fs)
+    G = torch.from_numpy(rng.standard_normal((B, F, n, 2))).float().cuda()
+    G = torch.view_as_complex(G)
+    got = torch.autograd.grad(y, x, G)[0]
+    xr = x.detach().double().requires_grad_(True)
+    yr = ref_forward(xr, sigma.detach().double(), freqs.detach().double(), fs, True)
+    want = torch.autograd.grad(yr, xr, G.to(torch.complex128))[0]
+    assert float(torch.linalg.vector_norm(got.double() - want)) <= 3.75e-7 * float(torch.linalg.vector_norm(want))
