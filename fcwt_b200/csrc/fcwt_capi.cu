@@ -219,6 +219,8 @@ bool encode_output_map16(void* base, int n, int M, int rows, CUtensorMap* map) {
 
 struct fcwt_plan;
 
+constexpr uint64_t kPlanPoolKeep = 128ull << 20;
+
 struct fcwt_context {
     int device = 0;
     cudaStream_t own = nullptr;
@@ -242,6 +244,11 @@ struct fcwt_context {
     // every live plan created on this context (cached or caller-owned): destroying
     // the context releases their device resources and detaches them
     std::vector<fcwt_plan*> plans;
+    // Memory of the plans (one block each). From cudaMalloc, a block of 1 to 10 MB took a
+    // mapping of its own, 0.4 ms and up to 40 ms on a busy host, where the small buffers of
+    // separate allocations had shared mappings; the pool maps 32 MB at a time, keeps at
+    // most kPlanPoolKeep of what closed plans gave back, and ends with the context.
+    cudaMemPool_t plan_pool = nullptr;
     // host-output pipeline: copy stream, per-slot "rows done" / "block copied" events
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t pipe_done[2] = {nullptr, nullptr}, pipe_copied[2] = {nullptr, nullptr};
@@ -299,7 +306,7 @@ struct fcwt_plan {
     DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, small_rows, tc_wts, tc_tabs;
     DevBuf tc_units;  // work list of the tensor-core engine (rows, the last ones possibly split)
     int n_units[2] = {0, 0};  // units of R = 16 and, after them, of R = 8
-    DevBuf mem;  // one allocation that holds the buffers plan_build fills
+    DevBuf mem;  // one block of the context's pool that holds the buffers plan_build fills
     int n_items = 0;
     int n_small = 0, small_log2L = 0;  // rows of N <= kMaxFusedN, log2 of their largest N / dec
     int n_rows = 0;
@@ -358,6 +365,8 @@ void plan_release(fcwt_plan* p) {
     p->sigs2.release();
     p->ds_tmp.release();
     p->shifted.release();
+    // (as with cudaFree, no stream may still use the block)
+    if (p->mem.p && cudaDeviceSynchronize() == cudaSuccess) cudaFreeAsync(p->mem.p, p->ctx->own);
     p->mem.release();
 }
 
@@ -728,7 +737,9 @@ int plan_build(fcwt_plan* P) {
         total += padded(want[i].second);
         if (i + 1 == n_filled) filled = total;
     }
-    FCWT_CUDA_TRY(P->mem.ensure(total));
+    void* block = nullptr;
+    FCWT_CUDA_TRY(cudaMallocFromPoolAsync(&block, total, ctx->plan_pool, st));
+    P->mem.part_of(block, total);
     size_t off = 0;
     for (auto& w : want) {
         w.first->part_of(P->mem.as<char>() + off, w.second);
@@ -1282,6 +1293,13 @@ int fcwt_context_create(int device, fcwt_context** out) {
     c->num_sms = prop.multiProcessorCount;
     cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMallocHost(&c->err_host, sizeof(int));
+    cudaMemPoolProps mp = {};
+    mp.allocType = cudaMemAllocationTypePinned;
+    mp.location.type = cudaMemLocationTypeDevice;
+    mp.location.id = device;
+    if (e == cudaSuccess) e = cudaMemPoolCreate(&c->plan_pool, &mp);
+    uint64_t keep = kPlanPoolKeep;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->plan_pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e == cudaSuccess) e = fcwt::engine_configure();
     if (e == cudaSuccess) e = fcwt::tc_configure();
     if (e == cudaSuccess) e = fcwt::small_configure();
@@ -1291,6 +1309,7 @@ int fcwt_context_create(int device, fcwt_context** out) {
     if (e != cudaSuccess) {
         if (c->own) cudaStreamDestroy(c->own);
         if (c->err_host) cudaFreeHost(c->err_host);
+        if (c->plan_pool) cudaMemPoolDestroy(c->plan_pool);
         delete c;
         return fail(FCWT_ERR_CUDA, std::string("context setup: ") + cudaGetErrorString(e));
     }
@@ -1342,6 +1361,8 @@ int fcwt_context_destroy(fcwt_context* ctx) {
         if (ctx->pipe_copied[i]) cudaEventDestroy(ctx->pipe_copied[i]);
     }
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+    cudaStreamSynchronize(ctx->own);
+    if (ctx->plan_pool) cudaMemPoolDestroy(ctx->plan_pool);
     if (ctx->own) cudaStreamDestroy(ctx->own);
     delete ctx;
     return FCWT_OK;
