@@ -220,6 +220,7 @@ bool encode_output_map16(void* base, int n, int M, int rows, CUtensorMap* map) {
 struct fcwt_plan;
 
 constexpr uint64_t kPlanPoolKeep = 128ull << 20;
+constexpr size_t kPlanPoolMax = 32ull << 20;
 
 struct fcwt_context {
     int device = 0;
@@ -247,7 +248,9 @@ struct fcwt_context {
     // Memory of the plans (one block each). From cudaMalloc, a block of 1 to 10 MB took a
     // mapping of its own, 0.4 ms and up to 40 ms on a busy host, where the small buffers of
     // separate allocations had shared mappings; the pool maps 32 MB at a time, keeps at
-    // most kPlanPoolKeep of what closed plans gave back, and ends with the context.
+    // most kPlanPoolKeep of what closed plans gave back, and ends with the context. Blocks
+    // over kPlanPoolMax are allocated by themselves: the pool would map and unmap them in
+    // parts (a plan of 48 channels: 96 ms to create instead of 91).
     cudaMemPool_t plan_pool = nullptr;
     // host-output pipeline: copy stream, per-slot "rows done" / "block copied" events
     cudaStream_t copy_stream = nullptr;
@@ -306,7 +309,7 @@ struct fcwt_plan {
     DevBuf pool, sigs, rows, items, fwd_jobs, fwd_tmp, graph_jobs, tc_rows, small_rows, tc_wts, tc_tabs;
     DevBuf tc_units;  // work list of the tensor-core engine (rows, the last ones possibly split)
     int n_units[2] = {0, 0};  // units of R = 16 and, after them, of R = 8
-    DevBuf mem;  // one block of the context's pool that holds the buffers plan_build fills
+    DevBuf mem;  // one block that holds the buffers plan_build fills: of the context's pool, or its own
     int n_items = 0;
     int n_small = 0, small_log2L = 0;  // rows of N <= kMaxFusedN, log2 of their largest N / dec
     int n_rows = 0;
@@ -366,7 +369,7 @@ void plan_release(fcwt_plan* p) {
     p->ds_tmp.release();
     p->shifted.release();
     // (as with cudaFree, no stream may still use the block)
-    if (p->mem.p && cudaDeviceSynchronize() == cudaSuccess) cudaFreeAsync(p->mem.p, p->ctx->own);
+    if (p->mem.p && !p->mem.own && cudaDeviceSynchronize() == cudaSuccess) cudaFreeAsync(p->mem.p, p->ctx->own);
     p->mem.release();
 }
 
@@ -737,9 +740,13 @@ int plan_build(fcwt_plan* P) {
         total += padded(want[i].second);
         if (i + 1 == n_filled) filled = total;
     }
-    void* block = nullptr;
-    FCWT_CUDA_TRY(cudaMallocFromPoolAsync(&block, total, ctx->plan_pool, st));
-    P->mem.part_of(block, total);
+    if (total <= kPlanPoolMax) {
+        void* block = nullptr;
+        FCWT_CUDA_TRY(cudaMallocFromPoolAsync(&block, total, ctx->plan_pool, st));
+        P->mem.part_of(block, total);
+    } else {
+        FCWT_CUDA_TRY(P->mem.ensure(total));
+    }
     size_t off = 0;
     for (auto& w : want) {
         w.first->part_of(P->mem.as<char>() + off, w.second);

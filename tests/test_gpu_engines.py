@@ -368,7 +368,7 @@ def test_wide_rows_of_several_chunks_per_item(fcwt, oracle, n, dec):
 def test_plan_memory_is_pooled_and_given_back(fcwt, oracle, monkeypatch):
     """Plans created beside living ones take no new device mapping each (that
     cost up to 40 ms a plan); closed plans leave at most 128 MB (in mappings of
-    32 MB) with the context, and nothing when the context ends."""
+    32 MB) with the context, a large one nothing, and all is free when it ends."""
     import torch
 
     from fcwt_b200 import _lib
@@ -377,17 +377,21 @@ def test_plan_memory_is_pooled_and_given_back(fcwt, oracle, monkeypatch):
         torch.cuda.synchronize()
         return torch.cuda.mem_get_info()[0]
 
-    fcwt.Plan(16384, oracle.scales(LOGSCALES, 1000, 2.0, 200.0, 96), fb=2.0).close()  # (kernels are loaded)
+    sc = oracle.scales(LOGSCALES, 1000, 2.0, 200.0, 96)
+    x = torch.randn(16384, device="cuda")
+    outs = [torch.empty((96, 16384), dtype=torch.complex64, device="cuda") for _ in range(8)]
+    warm = fcwt.Plan(16384, sc, fb=2.0)  # (loads the kernels, on the process's own context)
+    warm.execute(x, outs[0])
+    assert torch.equal(outs[0], outs[0].clone())
+    warm.close()
+    torch.cuda.empty_cache()
     free0 = free_bytes()
     ctx = _lib.Context(0)
     monkeypatch.setitem(_lib._contexts, 0, ctx)
-    sc = oracle.scales(LOGSCALES, 1000, 2.0, 200.0, 96)
     plans = [fcwt.Plan(16384, sc, fb=2.0)]
     free1 = free_bytes()
     plans += [fcwt.Plan(16384, sc, fb=2.0) for _ in range(7)]
     assert free_bytes() == free1
-    x = torch.randn(16384, device="cuda")
-    outs = [torch.empty((96, 16384), dtype=torch.complex64, device="cuda") for _ in plans]
     for p, o in zip(plans, outs):
         p.execute(x, o)
     for o in outs[1:]:
@@ -400,7 +404,6 @@ def test_plan_memory_is_pooled_and_given_back(fcwt, oracle, monkeypatch):
     assert free2 - free_bytes() <= 160 << 20
     for p in plans:
         p.close()
-    del x, outs
     torch.cuda.empty_cache()
     ctx.close()
     assert free0 - free_bytes() <= 4 << 20
