@@ -128,6 +128,14 @@ struct TuneChoice {
     int lag = 12;         // rows between a row's phase 1 and phase 2 items
     int engine = 0;       // 0: tensor-core engine for the rows it takes; 1: CUDA-core engine only
 };
+// Without a tuning file: 64 MB, and eight slots at least (with four, 30 rows of 2^22
+// waited for slots a sixth of the time, 3.56 against 2.89 ms). A file's budget is
+// kept to down to the four slots that the schedule needs.
+TuneChoice default_tune(int log2N) {
+    TuneChoice tc;
+    tc.scratch_mb = std::max(tc.scratch_mb, (int)((8ull * 8ull << log2N) >> 20));
+    return tc;
+}
 
 // Where a caller's pointer lives: 0 host memory (pageable or pinned), 1 memory
 // the kernels of device `dev` may use directly (that device's memory, or
@@ -627,9 +635,7 @@ int plan_build(fcwt_plan* P) {
         const TuneChoice& tc = ctx->tune[max_two_phase_log2N];
         const long long slot_elems = 1ll << max_two_phase_log2N;
         const int nt = (int)two_phase_rows.size();
-        // (8 slots at least: with 4, N = 2^22 waited for slots a sixth of the time, 3.56 against
-        // 2.89 ms for 30 rows)
-        int S = (int)std::max(8LL, std::min(40LL, ((long long)tc.scratch_mb << 20) / (slot_elems * 8)));
+        int S = (int)std::max(4LL, std::min(40LL, ((long long)tc.scratch_mb << 20) / (slot_elems * 8)));
         S = std::min(S, std::max(1, nt));
         int D = std::max(1, std::min(tc.lag, S / 2));
         if (S == 1) D = 1;
@@ -1321,6 +1327,7 @@ int fcwt_context_create(int device, fcwt_context** out) {
         return fail(FCWT_ERR_CUDA, std::string("context setup: ") + cudaGetErrorString(e));
     }
     *c->err_host = 0;
+    for (int i = 0; i <= fcwt::kMaxLog2N; i++) c->tune[i] = default_tune(i);
     c->stream = c->own;
     *out = c;
     return FCWT_OK;
@@ -2061,7 +2068,7 @@ int fcwt_create_optimization_plan(fcwt_context* ctx, int maxsize, int threads, i
     if (nt > fcwt::kMaxLog2N) return fail(FCWT_ERR_INVALID, "maxsize too large");
     for (int i = 11; i <= nt; i++) {
         const int N = 1 << i;
-        TuneChoice best;
+        TuneChoice best = default_tune(i);
         if (level > 0 && N > fcwt::kMaxFusedN) {
             // candidate grid grows with the level
             std::vector<TuneChoice> cands;
@@ -2071,7 +2078,7 @@ int fcwt_create_optimization_plan(fcwt_context* ctx, int maxsize, int threads, i
             // CUDA-core engine: scratch budget x lag grid; tensor-core engine: one candidate
             for (int a = 0; a < nm; a++)
                 for (int b = 0; b < nm; b++) cands.push_back({mbs[a + (4 - nm)], lags[b], 1});
-            if (N >= fcwt::kTcMinN) cands.push_back(TuneChoice{});
+            if (N >= fcwt::kTcMinN) cands.push_back(default_tune(i));
             // synthetic workload: N samples, 256 log-spaced scales over the band
             const int fn = 256;
             std::vector<float> sc((size_t)fn), x((size_t)N);

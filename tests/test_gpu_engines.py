@@ -407,3 +407,36 @@ def test_plan_memory_is_pooled_and_given_back(fcwt, oracle, monkeypatch):
     torch.cuda.empty_cache()
     ctx.close()
     assert free0 - free_bytes() <= 4 << 20
+
+
+def test_tuning_file_bounds_the_scratch_ring(fcwt, oracle, monkeypatch, tmp_path):
+    """A tuning file's scratch budget holds down to four rows (64 MB at
+    N = 2^21): the context that loads 16 MB takes 192 MB less device memory for the
+    same wide rows than one that loads 256 MB (16 rows), with the same bits."""
+    import ctypes
+
+    import torch
+
+    from fcwt_b200 import _lib
+
+    n, fn = 1 << 21, 20
+    sc = oracle.scales(LINFREQS, 1000, 300.0, 480.0, fn)
+    x = torch.from_numpy(np.random.default_rng(3).standard_normal(n).astype(np.float32)).cuda()
+    out = torch.empty((fn, n), dtype=torch.complex64, device="cuda")
+    used, first = {}, None
+    for mb in (16, 16, 256):  # (the first one loads the kernels)
+        (tmp_path / f"n{n}_t1.wis").write_text(f"fcwt-b200-tune 1\nN {n}\nthreads 1\nscratch_mb {mb}\nlag 4\nengine 1\n")
+        ctx = _lib.Context(0)
+        monkeypatch.setitem(_lib._contexts, 0, ctx)
+        _lib.call("fcwt_load_optimization_plan", ctx.handle, n, 1, ctypes.c_char_p(str(tmp_path).encode()))
+        plan = fcwt.Plan(n, sc, fb=6.0)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        plan.execute(x, out)
+        ctx.synchronize()
+        used[mb] = before - torch.cuda.mem_get_info()[0]
+        assert first is None or torch.equal(out, first)
+        first = out.clone()
+        plan.close()
+        ctx.close()
+    assert used[256] - used[16] >= 180 << 20
