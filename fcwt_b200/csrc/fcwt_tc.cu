@@ -677,6 +677,24 @@ __device__ __forceinline__ void finish_pair(const Cx (&x)[16], uint32_t tw, char
     }
 }
 
+// finish_pair for the row's length: N' / 16 = 2^logS samples are between consecutive a2,
+// logS = 9 or 10 for R = 8 and 10 to 19 for R = 16. Up to 16 the 15 steps of 8 bytes fit
+// the 24-bit offset of a store (500000 x 300: 328 us, its power 295; with the steps added
+// to the addresses 335 and 333). Longer rows add them.
+template <int OT, int LO, int HI>
+__device__ __forceinline__ void store_pair(const Cx (&x)[16], uint32_t tw, char* pa, char* pb, int la, int lb,
+                                           int logS) {
+    if constexpr (LO == HI) {
+        finish_pair<OT, LO <= 16 ? LO : 0>(x, tw, pa, pb, la, lb, logS);
+    } else {
+        constexpr int MID = (LO + HI) / 2;
+        if (logS <= MID)
+            store_pair<OT, LO, MID>(x, tw, pa, pb, la, lb, logS);
+        else
+            store_pair<OT, MID + 1, HI>(x, tw, pa, pb, la, lb, logS);
+    }
+}
+
 // One unit: a row's descriptors, its tiles and the scale of its Z.
 struct UnitSlot {
     int idx;    // position in the queue; at or past the end: stop
@@ -1018,15 +1036,7 @@ __device__ __forceinline__ void consume(const TcParams& P, TcShared& sh, unsigne
                 if (c >= G.M) la = lb = 0;
                 char* pa = outb + (size_t)((unsigned)ta * ES);
                 char* pb = outb + (size_t)((unsigned)tb * ES);
-                switch (logS) {
-                    case 10: finish_pair<OT, 10>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                    case 11: finish_pair<OT, 11>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                    case 12: finish_pair<OT, 12>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                    case 13: finish_pair<OT, 13>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                    case 14: finish_pair<OT, 14>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                    case 16: finish_pair<OT, 16>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                    default: finish_pair<OT, 0>(x, tp + 64u, pa, pb, la, lb, logS); break;
-                }
+                store_pair<OT, R == 16 ? 10 : 9, R == 16 ? 17 : 10>(x, tp + 64u, pa, pb, la, lb, logS);
                 __syncwarp();
             }
         }

@@ -440,3 +440,33 @@ def test_tuning_file_bounds_the_scratch_ring(fcwt, oracle, monkeypatch, tmp_path
         plan.close()
         ctx.close()
     assert used[256] - used[16] >= 180 << 20
+
+
+# N' / 16 = 2^9 (128-bin blocks, half a tile) and 2^15 .. 2^18 samples between the outputs
+# of a thread: the largest that a store's offset holds is 2^16
+@pytest.mark.parametrize("n,dec", [(8193 * 2, 4), (262145, 1), (524288, 1), (524289, 1), (1 << 20, 2), (1 << 21, 1), (2097153, 1)])
+@pytest.mark.parametrize("half", [False, True])
+def test_store_addressing_by_length(fcwt, oracle, n, dec, half):
+    """Rows of the lengths whose store offsets differ, complex64 within the 3.6e-6
+    of 2^-21 per product and 51 FP32 roundings of 2^-24, float16 within its own
+    2^-11 per part besides."""
+    import torch
+
+    fn = 4
+    # bands of at most 62 blocks of the window, wherever the length is
+    sc = fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LOGSCALES, 100000, 100000 * 1000.0 / n, 100000 * 3000.0 / n, fn)
+    x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    plan = fcwt.Plan(n, sc, fb=2.0, norm=True, time_stride=dec)
+    assert plan.stats()["tensor_core_rows"] == fn
+    if half:
+        out = torch.full((*plan.out_shape, 2), float("nan"), dtype=torch.float16, device="cuda")
+        plan.execute(torch.from_numpy(x).cuda(), out, out_type=fcwt.FCWT_OUT_F16)
+        got = torch.view_as_complex(out.float()).cpu().numpy()
+    else:
+        out = torch.full(plan.out_shape, float("nan"), dtype=torch.complex64, device="cuda")
+        plan.execute(torch.from_numpy(x).cuda(), out)
+        got = out.cpu().numpy()
+    plan.close()
+    ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)[:, ::dec]
+    for r in range(fn):
+        assert rel_l2(got[r], ref[r]) <= 3.6e-6 + (2.0 ** -11 if half else 0.0), r
