@@ -841,8 +841,10 @@ __device__ __forceinline__ void produce(const TcParams& P, TcShared& sh, unsigne
                 prod_bar();
             }
             if (atab != acur) {
-                mma_done(t - 1);
+                // (the copying thread alone waits: another, held up until the issuers are through
+                // with the unit, would find the barrier two phases on and wait for a third)
                 if (ptid == 0) {
+                    mma_done(t - 1);
                     load_a(a0, atab, kTcColBytes, smem_u32(&sh.abar));
                     free_all();
                     load_col(a0, atab, kTcColBytes, smem_u32(&sh.abar));
