@@ -643,7 +643,10 @@ int plan_build(fcwt_plan* P) {
         // Points per item: 16384 when that leaves 8 items per CTA, else one chunk (8 or 64
         // k2, 8 columns; finer items end more evenly). An item's claim, waits and signal
         // are a few microseconds in which most of the CTA stands still. 305 rows of 2^20:
-        // 3.15 -> 2.98 ms. Items larger than that would outrun the scratch ring.
+        // 3.15 -> 2.98 ms. But the items of D rows are at least one per CTA: with fewer, the
+        // items in flight span more rows than the lag, and a phase-2 item waits for a phase 1
+        // that still runs. (3000 rows of 16384 2.14 ms with 16384 points each, 1.34 with this
+        // rule; of 131072 3.14 and 2.65; one chunk per item before: 1.37 and 2.60.)
         long long points = 0;
         for (int g : two_phase_rows) points += P->sig[(size_t)rows[(size_t)g].sig].sp.N;
         const long long target = points >= 16384ll * 8 * ctx->engine_ctas ? 16384 : 0;
@@ -659,10 +662,18 @@ int plan_build(fcwt_plan* P) {
             d.slot = i % S;
             d.wait_row = i >= S ? two_phase_rows[(size_t)(i - S)] : -1;
             const int k2s = d.K > kMaxK ? kWideChunk : kChunk;
-            ca[(size_t)i] = per_item((long long)k2s * M, kP2 / k2s);
-            cb[(size_t)i] = per_item((long long)kGroupCols * kP2, M / d.dec / kGroupCols);
-            d.n_a = kP2 / k2s / ca[(size_t)i];
-            d.n_b = M / d.dec / kGroupCols / cb[(size_t)i];
+            int& a = ca[(size_t)i];
+            int& b = cb[(size_t)i];
+            a = per_item((long long)k2s * M, kP2 / k2s);
+            b = per_item((long long)kGroupCols * kP2, M / d.dec / kGroupCols);
+            while ((kP2 / k2s / a + M / d.dec / kGroupCols / b) * D < ctx->engine_ctas && (a > 1 || b > 1)) {
+                if (b == 1 || (a > 1 && (long long)a * k2s * M >= (long long)b * kGroupCols * kP2))
+                    a /= 2;
+                else
+                    b /= 2;
+            }
+            d.n_a = kP2 / k2s / a;
+            d.n_b = M / d.dec / kGroupCols / b;
         }
         for (int step = 0; step < nt + D; step++) {
             if (step < nt) {

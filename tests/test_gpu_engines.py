@@ -470,3 +470,32 @@ def test_store_addressing_by_length(fcwt, oracle, n, dec, half):
     ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True)[:, ::dec]
     for r in range(fn):
         assert rel_l2(got[r], ref[r]) <= 3.6e-6 + (2.0 ** -11 if half else 0.0), r
+
+
+def test_items_do_not_outgrow_the_lag(fcwt, ctx):
+    """The CUDA-core engine takes larger work items for many rows. Rows of 16384
+    samples get none so large that the items in flight span more rows than the
+    lag between the phases: 3000 rows take at most 1.9 times as long as 2000
+    (1.5 by their number; 2.3 when items waited for the rows before them)."""
+    import torch
+
+    from fcwt_b200 import _lib
+
+    ctx.set_engine(_lib.FCWT_ENGINE_CUDA_CORES)
+    n = 16384
+    x = torch.randn(n, device="cuda")
+    ms = {}
+    for fn in (2000, 3000):
+        plan = fcwt.Plan(n, fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LINFREQS, 1000, 1.0, 101.0, fn), fb=2.0)
+        out = torch.empty((fn, n), dtype=torch.complex64, device="cuda")
+        times = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            plan.execute(x, out)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        ms[fn] = sorted(times)[3]
+        plan.close()
+    assert ms[3000] <= 1.9 * ms[2000], ms
