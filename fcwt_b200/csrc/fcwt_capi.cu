@@ -125,8 +125,11 @@ struct DevBuf {
 // Scheduling choices of the two-phase row engine for one padded length.
 struct TuneChoice {
     int scratch_mb = 64;  // budget of the scratch ring
-    int lag = 12;         // rows between a row's phase 1 and phase 2 items
+    int lag = 20;         // rows between a row's phase 1 and phase 2 items: a CTA holds its next
+                          // item while it runs one, so the items in flight are two per CTA (1000
+                          // rows of 65536 0.54 ms, of 16384 3000 rows 1.06; with 12 0.70 and 1.34)
     int engine = 0;       // 0: tensor-core engine for the rows it takes; 1: CUDA-core engine only
+    bool given = false;   // by a tuning file or the tuner
 };
 // Without a tuning file: 64 MB, and eight slots at least (with four, 30 rows of 2^22
 // waited for slots a sixth of the time, 3.56 against 2.89 ms). A file's budget is
@@ -635,21 +638,25 @@ int plan_build(fcwt_plan* P) {
         const TuneChoice& tc = ctx->tune[max_two_phase_log2N];
         const long long slot_elems = 1ll << max_two_phase_log2N;
         const int nt = (int)two_phase_rows.size();
-        int S = (int)std::max(4LL, std::min(40LL, ((long long)tc.scratch_mb << 20) / (slot_elems * 8)));
+        // decimated rows have fewer phase-2 items, so more of them are in flight: 128 MB (every
+        // 4th sample of 100 wide rows of 2^20 0.84 ms with 64 MB, 0.79)
+        const bool decimated = nsig == 1 && P->sig[0].dec > 1;
+        const long long mb = decimated && !tc.given ? std::max(tc.scratch_mb, 128) : tc.scratch_mb;
+        int S = (int)std::max(4LL, std::min(40LL, (mb << 20) / (slot_elems * 8)));
         S = std::min(S, std::max(1, nt));
         int D = std::max(1, std::min(tc.lag, S / 2));
         if (S == 1) D = 1;
         if (D >= S && S > 1) return fail(FCWT_ERR_INVALID, "internal: lag >= slots");
-        // Points per item: 16384 when that leaves 8 items per CTA, else one chunk (8 or 64
-        // k2, 8 columns; finer items end more evenly). An item's claim, waits and signal
+        // Points per item: up to 16384 while that leaves 8 items per CTA, and one chunk at least
+        // (8 or 64 k2, 8 columns; finer items end more evenly). An item's claim, waits and signal
         // are a few microseconds in which most of the CTA stands still. 305 rows of 2^20:
-        // 3.15 -> 2.98 ms. But the items of D rows are at least one per CTA: with fewer, the
-        // items in flight span more rows than the lag, and a phase-2 item waits for a phase 1
-        // that still runs. (3000 rows of 16384 2.14 ms with 16384 points each, 1.34 with this
-        // rule; of 131072 3.14 and 2.65; one chunk per item before: 1.37 and 2.60.)
+        // 3.15 -> 2.98 ms; 200 wide rows of 131072 0.64 ms with single chunks of 1024, 0.54 now.
+        // But the items of D rows are at least one per CTA: with fewer, the items in flight span
+        // more rows than the lag, and a phase-2 item waits for a phase 1 that still runs (3000
+        // rows of 16384: 2.14 ms with 16384 points each and a lag of 12, 1.34 with this rule).
         long long points = 0;
         for (int g : two_phase_rows) points += P->sig[(size_t)rows[(size_t)g].sig].sp.N;
-        const long long target = points >= 16384ll * 8 * ctx->engine_ctas ? 16384 : 0;
+        const long long target = std::min(16384ll, points / (8ll * ctx->engine_ctas));
         auto per_item = [&](long long chunk_points, int chunks) {
             int c = 1;
             while (2 * c <= chunks && 2 * c * chunk_points <= target) c *= 2;
@@ -2039,6 +2046,7 @@ int fcwt_load_optimization_plan(fcwt_context* ctx, int n, int threads, const cha
     std::getline(f, magic);
     if (magic != "fcwt-b200-tune 1") return fail(FCWT_ERR_IO, "optimization plan '" + path + "' is malformed");
     TuneChoice tc;
+    tc.given = true;
     std::string line;
     int got = 0;
     while (std::getline(f, line)) {
@@ -2084,11 +2092,11 @@ int fcwt_create_optimization_plan(fcwt_context* ctx, int maxsize, int threads, i
             // candidate grid grows with the level
             std::vector<TuneChoice> cands;
             const int mbs[] = {16, 32, 64, 96};
-            const int lags[] = {4, 8, 12, 16};
+            const int lags[] = {20, 16, 12, 8};
             const int nm = level == 1 ? 2 : (level == 2 ? 3 : 4);
             // CUDA-core engine: scratch budget x lag grid; tensor-core engine: one candidate
             for (int a = 0; a < nm; a++)
-                for (int b = 0; b < nm; b++) cands.push_back({mbs[a + (4 - nm)], lags[b], 1});
+                for (int b = 0; b < nm; b++) cands.push_back({mbs[a + (4 - nm)], lags[b], 1, true});
             if (N >= fcwt::kTcMinN) cands.push_back(default_tune(i));
             // synthetic workload: N samples, 256 log-spaced scales over the band
             const int fn = 256;

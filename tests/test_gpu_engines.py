@@ -499,3 +499,29 @@ def test_items_do_not_outgrow_the_lag(fcwt, ctx):
         ms[fn] = sorted(times)[3]
         plan.close()
     assert ms[3000] <= 1.9 * ms[2000], ms
+
+
+# items of 1, 2, 4 and 8 chunks of 8 k2 and, decimated, of several column groups
+@pytest.mark.parametrize("n,dec,fn", [(131072, 1, 40), (131071, 1, 90), (131072, 1, 200), (262143, 2, 150), (262144, 16, 200)])
+def test_wide_rows_item_sizes(fcwt, oracle, ctx, n, dec, fn):
+    """Wide rows of the CUDA-core engine in work items of the sizes that the
+    number of rows gives. Bound: 2 x 18 butterfly levels of 2^-24 and 10
+    twiddles of 2^-22: 4.6e-6 if all were to add up."""
+    import torch
+
+    from fcwt_b200 import _lib
+
+    ctx.set_engine(_lib.FCWT_ENGINE_CUDA_CORES)
+    rows = [0, fn // 2, fn - 1]
+    sc = fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LINFREQS, 1000, 150.0, 450.0, fn)
+    x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    plan = fcwt.Plan(n, sc, fb=2.0, time_stride=dec)
+    assert plan.stats()["tensor_core_rows"] == 0
+    out = torch.full(plan.out_shape, float("nan"), dtype=torch.complex64, device="cuda")
+    plan.execute(torch.from_numpy(x).cuda(), out)
+    got = out[rows].cpu().numpy()
+    assert not bool(torch.isnan(torch.view_as_real(out)).any())
+    plan.close()
+    ref = oracle.cwt_fp64(x, sc.scales, 2.0, 1, True, rows=rows)[:, ::dec]
+    for r in range(len(rows)):
+        assert rel_l2(got[r], ref[r]) <= 4.6e-6, rows[r]
