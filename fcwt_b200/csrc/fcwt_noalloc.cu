@@ -103,9 +103,18 @@ struct PoolCopy {
 };
 static_assert(sizeof(RowCopy) <= 32000 && sizeof(PoolCopy) <= 32000, "kernel parameter limit");
 
-__global__ void k_na_rows(const __grid_constant__ RowCopy c, RowDesc* __restrict__ dst, SigDesc* __restrict__ dsig) {
-    for (int i = threadIdx.x; i < c.count; i += blockDim.x) dst[c.first + i] = c.rows[i];
-    if (c.write_sig && threadIdx.x == 0) *dsig = c.sig;
+// Parameters are read through the constant cache, one address at a time: each thread
+// copies a word of 8 bytes, spread over the SMs. (With a row per thread of one CTA, whose
+// lanes read 136 bytes apart, a launch of 232 rows took 43 us.)
+constexpr int kRowWords = (int)(sizeof(RowDesc) / sizeof(uint2));
+constexpr int kRowCopyThreads = 128;
+static_assert(sizeof(RowDesc) % sizeof(uint2) == 0, "rows are copied in words of 8 bytes");
+__global__ void __launch_bounds__(kRowCopyThreads)
+    k_na_rows(const __grid_constant__ RowCopy c, RowDesc* __restrict__ dst, SigDesc* __restrict__ dsig) {
+    const int i = blockIdx.x * kRowCopyThreads + threadIdx.x;
+    if (i < c.count * kRowWords)
+        reinterpret_cast<uint2*>(dst + c.first)[i] = reinterpret_cast<const uint2*>(c.rows)[i];
+    if (c.write_sig && i == 0) *dsig = c.sig;
 }
 
 __global__ void k_na_pool(const __grid_constant__ PoolCopy c, float* __restrict__ dst) {
@@ -287,7 +296,8 @@ extern "C" int fcwt_cwt_noalloc(const float* input, int n, float fb, const float
             c.count = std::min(kRowsPerCopy, fn - r0);
             c.write_sig = r0 == 0;
             std::memcpy(c.rows, rows.data() + r0, sizeof(RowDesc) * (size_t)c.count);
-            k_na_rows<<<1, 256, 0, st>>>(c, drows, dsig);
+            k_na_rows<<<(c.count * kRowWords + kRowCopyThreads - 1) / kRowCopyThreads, kRowCopyThreads, 0, st>>>(c, drows,
+                                                                                                              dsig);
             NA_TRY(cudaGetLastError());
         }
         static thread_local PoolCopy pc_buf;

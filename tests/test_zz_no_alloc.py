@@ -98,3 +98,27 @@ def test_noalloc_rejects_a_device_scales_array():
                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.byref(status))
     assert rc == _lib.FCWT_ERR_INVALID
     assert b"host" in lib.fcwt_last_error()
+
+
+@pytest.mark.parametrize("n", [100, 9000])
+@pytest.mark.parametrize("fn", [1, 15, 232, 233, 465, 1024])
+def test_noalloc_row_descriptors(n, fn):
+    """Every row arrives, for row counts at the edges of the descriptor copies
+    (232 rows each, 128 words of 8 bytes per CTA): the result equals the
+    allocating call's within the two paths' rounding."""
+    import torch
+
+    import fcwt_b200 as fcwt
+    from fcwt_b200 import _lib
+
+    sc = fcwt.Scales(fcwt.Morlet(2.0), fcwt.FCWT_LINFREQS, 1000, 20.0, 200.0, fn).scales
+    x = torch.from_numpy(np.random.default_rng(fn).standard_normal(n).astype(np.float32)).cuda()
+    got = torch.full((fn, n), float("nan"), dtype=torch.complex64, device="cuda")
+    rc, st = _noalloc(_lib.load(), x, sc, 2.0, 1, True, got)
+    assert rc == 0 and st == 0
+    want = torch.empty_like(got)
+    fcwt.FCWT(fcwt.Morlet(2.0), 1, False, True).cwt(x, sc, want)
+    torch.cuda.synchronize()
+    g, w = got.cpu().numpy(), want.cpu().numpy()
+    for r in range(fn):
+        assert rel_l2(g[r], w[r]) < TOL, r
