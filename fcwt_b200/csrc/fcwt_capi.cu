@@ -472,10 +472,10 @@ std::vector<int> plan_tc_units(const std::vector<int>& tc_rows, const std::vecto
     return best;
 }
 
-// Builds descriptors and the work list of all signals. Rows of N < 1024 get a
-// direct-DFT item, rows of N <= 8192 one fused item; two-phase rows (all
-// signals, in order) get phase-1 items and phase-2 items, phase 2 of row r
-// issued after phase 1 of row r + lag, scratch slots reused round-robin.
+// Builds descriptors and the work lists of all signals. Rows of N <= kMaxFusedN run
+// whole, one CTA each; rows whose window fits are units of the tensor-core engine; the
+// others (two-phase rows, all signals, in order) get phase-1 items and phase-2 items,
+// phase 2 of row r issued after phase 1 of row r + lag, scratch slots reused round-robin.
 int plan_build(fcwt_plan* P) {
     using namespace fcwt;
     fcwt_context* ctx = P->ctx;

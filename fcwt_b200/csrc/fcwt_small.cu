@@ -9,10 +9,10 @@
 //
 // Few rows are bound by serial latency (launch, descriptors, bins, three or four
 // stages), so there is no work queue and no table is computed in the prologue; many
-// rows of N = 8192 by one CTA per SM (128 registers). On the work queue of the
-// persistent engine (claim, item, row, signal, 16 input chunks, one warp's column DFT
-// in turn) a whole call took: 64 rows of N = 1024 50 us, now 26; 2000 rows of 2048
-// 124, now 63; of 4096 151, now 94; of 8192 215, now 187; of 8192 by 4 203, now 84.
+// rows of N = 8192 by one CTA per SM (512 threads of 128 registers). On the work queue of
+// the persistent engine (claim, item, row, signal, 16 input chunks, one warp's column DFT
+// in turn) a whole call took: 64 rows of 1000 samples 50 us, now 12; 2000 rows of 2048
+// 121, now 44; 1000 of 4096 92, now 48; 1000 of 8192 130, now 97.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -34,7 +34,7 @@ __device__ __forceinline__ int small_pos(int i) { return i + (i >> 4); }
 
 // One radix-R stage in place: every thread takes its inputs into registers (at most
 // 16 values: blockDim >= L / 16), the CTA waits, and the results go to their places.
-// In place a row of 8192 takes 70 KB, so that three of them share an SM.
+// In place a row of 8192 takes 70 KB instead of 139.
 template <int R>
 __device__ __forceinline__ void small_stage(float2* __restrict__ a, int log2L, int log2Ns, const float2* __restrict__ tw,
                                             int log2N, const float2* __restrict__ ts) {
